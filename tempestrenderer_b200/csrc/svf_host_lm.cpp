@@ -314,11 +314,9 @@ svf_status launch_lm(svf_ctx* ctx, Layout* lay, const svf_lsq_options* o, const 
     lm_fault_injection(a);
     SVF_CUDA(cudaMemsetAsync(ctx->counter.p, 0, 16, ctx->stream));   // the error words are zeroed per call
     a.rgb = r.rgb ? 1u : 0u;
-    int per_sm = svf::lm_max_ctas_per_sm(a.L, a.lum_stride, c, r.rgb);
-    if(per_sm <= 0)
+    if(svf::lm_max_ctas_per_sm(a.L, a.lum_stride, c, r.rgb) <= 0)
         return fail(SVF_EINVAL, "the LM kernel (%d threads) does not fit on an SM for L = %u", c.threads, a.L);
-    uint64_t grid = std::min<uint64_t>((uint64_t)per_sm * ctx->sms, r.texels);
-    SVF_CUDA(svf::launch_lm_fit(a, c, (int)std::max<uint64_t>(grid, 1), ctx->stream));
+    SVF_CUDA(svf::launch_lm_fit(a, c, ctx->sms, ctx->stream));
     return SVF_OK;
 }
 

@@ -62,6 +62,7 @@ struct LmArgs
     uint32_t rgb;              // the 11-parameter RGB fit (svf_lm.cu RgbModel)
     LmConfig cfg;
     uint32_t* work_counter;    // zeroed before the launch
+    uint32_t counter_base;     // texels dealt to the slots before the counter is used (set by launch_lm_fit)
     uint32_t* error_flag;      // set non-zero by a bounded wait that expired
     // Fault injection for tests (the host sets it from the environment): the slab
     // copy of texel fault_skip_texel is not issued, so its wait runs out;
@@ -86,7 +87,7 @@ LmKernelChoice lm_default_choice(uint32_t L, uint64_t lum_stride, bool rgb = fal
 int            lm_candidates(uint32_t L, LmKernelChoice* out, int max);
 size_t         lm_smem_bytes(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool rgb = false);
 int            lm_max_ctas_per_sm(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool rgb = false);
-cudaError_t    launch_lm_fit(const LmArgs& args, LmKernelChoice c, int grid, cudaStream_t stream);
+cudaError_t    launch_lm_fit(const LmArgs& args, LmKernelChoice c, int sms, cudaStream_t stream);   // sms: of the device
 
 // svf_lsq_fit_batch_noalloc: repack, geometry and LM on `stream` with the
 // library's static device scratch array; waits for the stream.  flags[0]: the

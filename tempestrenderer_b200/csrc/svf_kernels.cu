@@ -691,11 +691,7 @@ cudaError_t launch_lm_fit_noalloc(const float* lights_parabolic, uint32_t L, con
     a.fault_skip_texel = kLmNoFault;
     a.wait_spins = 0;
     const LmKernelChoice choice = lm_default_choice(L, stride);
-    const int per_sm = lm_max_ctas_per_sm(L, stride, choice);
-    if(per_sm <= 0)
-        return cudaErrorInvalidConfiguration;
-    const uint64_t grid = std::min<uint64_t>((uint64_t)per_sm * sms, texels);
-    if((e = launch_lm_fit(a, choice, (int)std::max<uint64_t>(grid, 1), stream)) != cudaSuccess)
+    if((e = launch_lm_fit(a, choice, sms, stream)) != cudaSuccess)
         return e;
     if(stats)
     {

@@ -122,6 +122,13 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+__device__ __forceinline__ uint64_t global_ns()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Bounded wait for phase `parity` of `bar` (at most `spins` polls, 0: the
 // default bound); false when the bound expired.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t spins = 0)
@@ -566,6 +573,20 @@ __device__ __forceinline__ double warp_sum(double x)
     return x;
 }
 
+__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "sub.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
 // Symmetric pair evaluation.  For the two ordered pairs of one unordered pair
 // {a, b} (light b seen from view a, and light a seen from view b) the
 // specular core is the same: s = a_a + a_b, Q, S = sp_a + sp_b, g = |s|^2 and
@@ -588,6 +609,9 @@ __device__ __forceinline__ double warp_sum(double x)
 // entry of a is a broadcast), consecutive lights b (distinct banks), slab
 // elements a L + b (consecutive) and b L + a (stride L: distinct banks for
 // odd L).
+//
+// LumPass::add below is the same without a Fresnel factor in the paired
+// instructions.
 template <bool kFresnel, bool kAllUp>
 __device__ __forceinline__ void sym_pair(const PassConst& c, const Entry& ea, const Entry& eb, float refr, float y1,
                                          float y2, float wt1, float wt2, float* acc, double& r2)
@@ -674,26 +698,160 @@ __device__ __forceinline__ void sym_pair(const PassConst& c, const Entry& ea, co
     }
 }
 
+
+// The luminance fit without a Fresnel factor: sym_pair's operations, operation
+// for operation, two of one pair's values to an instruction where they come in
+// twos (add/mul/fma .f32x2).  A pass is bound by the issue slots, not by the
+// FP32 lanes: the scalar form issued about 150 instructions a step, 35 of them
+// the sums' FMAs, and kept the FP32 pipe 55 % busy; a paired FMA does two of the
+// sums in one slot and rounds each half as the scalar FMA does, so the results
+// are the same bits.  (Pairing two direction pairs instead, worker_pass2, needs
+// 35 paired sums and twice the entries: too many registers.)
+// The products are contracted as written here, whatever the compiler would
+// choose: a b + c d is fma(a, b, c d).  With A = (V0, V1), B = (V4, V5),
+// C = (V6, V2) the sums are the rows of J^T J taken two columns at a time.
+struct LumSums
+{
+    float2 h0A, h0B, h0C, h1B, h1C, h2B, h2C, h4B, h45_6;   // PV_i times A, B, C; (PV4, PV5) V6
+    float2 xA, xB, xC, rA, rB, rC, zu;                      // the diffuse column, J^T r, (H33, g3)
+    float h11, h55, h66;
+
+    __device__ __forceinline__ void clear()
+    {
+        h0A = h0B = h0C = h1B = h1C = h2B = h2C = h4B = h45_6 = f2(0.0f);
+        xA = xB = xC = rA = rB = rC = zu = f2(0.0f);
+        h11 = h55 = h66 = 0.0f;
+    }
+
+    // in the order of the scalar sums: the upper J^T J, then J^T r
+    __device__ __forceinline__ void unpack(float* acc) const
+    {
+        auto put = [&](int i, int j, float v) { acc[hix<kParams>(i, j)] = v; };
+        put(0, 0, h0A.x); put(0, 1, h0A.y); put(0, 4, h0B.x); put(0, 5, h0B.y); put(0, 6, h0C.x); put(0, 2, h0C.y);
+        put(1, 1, h11);   put(1, 4, h1B.x); put(1, 5, h1B.y); put(1, 6, h1C.x); put(1, 2, h1C.y);
+        put(2, 4, h2B.x); put(2, 5, h2B.y); put(2, 6, h2C.x); put(2, 2, h2C.y);
+        put(4, 4, h4B.x); put(4, 5, h4B.y); put(4, 6, h45_6.x); put(5, 6, h45_6.y);
+        put(5, 5, h55);   put(6, 6, h66);
+        put(0, 3, xA.x);  put(1, 3, xA.y);  put(3, 4, xB.x);  put(3, 5, xB.y);  put(3, 6, xC.x);  put(2, 3, xC.y);
+        put(3, 3, zu.x);
+        float* g = acc + kHessian;
+        g[0] = rA.x; g[1] = rA.y; g[2] = rC.y; g[3] = zu.y; g[4] = rB.x; g[5] = rB.y; g[6] = rC.x;
+    }
+};
+
+// A pass's constants, in registers.
+struct LumPass
+{
+    float u, v, ks, kd, ks_on, kd_on, t2c;
+    float2 uv4, rs, t10c, om0, om1, om2;   // (4u, 4v), (1/sx, 1/sy), (1 - u, v - 1), om columns of e0, e1
+
+    __device__ __forceinline__ explicit LumPass(const PassConst& c)
+    {
+        u = c.u;
+        v = c.v;
+        ks = c.ks;
+        kd = c.kd;
+        ks_on = c.ks_on;
+        kd_on = c.kd_on;
+        uv4 = make_float2(4.0f * c.u, 4.0f * c.v);
+        rs = make_float2(c.rsx, c.rsy);
+        t10c = make_float2(1.0f - c.u, c.v - 1.0f);
+        t2c = c.u - c.v;
+        // (the rate of e2 is the body z axis, (0, 0, 1): its dq is t2)
+        om0 = make_float2(c.om[0], c.om[3]);
+        om1 = make_float2(c.om[1], c.om[4]);
+        om2 = make_float2(c.om[2], c.om[5]);
+    }
+
+    // One unordered pair {a, b}: table entries x (a) and y (b) of the core0,
+    // core1 and deriv arrays, samples y1 (view a, light b) and y2 (view b, light
+    // a), weights wt1, wt2 (0 or 1).
+    template <bool kAllUp, bool kGuard>
+    __device__ __forceinline__ void add(const float4& x0, const float4& x1, const float4& x2, const float4& y0,
+                                        const float4& y1v, const float4& y2v, float y1, float y2, float wt1, float wt2,
+                                        LumSums& a, double& r2) const
+    {
+        const float2 s01 = add2(make_float2(x0.x, x0.y), make_float2(y0.x, y0.y));
+        const float2 s2S = add2(make_float2(x0.z, x0.w), make_float2(y0.z, y0.w));
+        const float s2 = s2S.x, S = s2S.y;
+        const float2 q01 = mul2(s01, s01);
+        const float g = __fmaf_rn(s2, s2, __fadd_rn(q01.x, q01.y));
+        const float Q = __fmaf_rn(s2, s2, __fmaf_rn(u, q01.x, __fmul_rn(v, q01.y)));
+        const float QQ = __fmul_rn(Q, Q), QQS = __fmul_rn(QQ, S);
+        const float rden = QQS > 1e-37f ? rcp_approx(QQS) : 0.0f;
+        const float C = __fmul_rn(__fmul_rn(g, g), rden);
+        // x1, y1v: (kspec kv, up, kdc, dsp4)
+        float w1 = x1.x, w2 = __fmul_rn(wt2, y1v.x), h1 = y1v.z, h2 = wt2;
+        if(kGuard)
+            w1 = __fmul_rn(wt1, w1);
+        if(kAllUp)
+        {
+            if(kGuard)
+                h1 = __fmul_rn(wt1, h1);
+        }
+        else
+        {
+            w1 = __fmul_rn(w1, y1v.y);
+            w2 = __fmul_rn(w2, x1.y);
+            h1 = __fmul_rn(kGuard ? __fmul_rn(wt1, x1.y) : x1.y, h1);
+            h2 = __fmul_rn(h2, y1v.y);
+        }
+        h2 = __fmul_rn(h2, x1.z);
+        const float sp1 = __fmul_rn(w1, C), sp2 = __fmul_rn(w2, C);
+        const float r1 = __fsub_rn(y1, __fmaf_rn(kd, h1, __fmul_rn(ks, sp1)));
+        const float rb = __fsub_rn(y2, __fmaf_rn(ks, sp2, __fmul_rn(kd, h2)));
+        r2 = fma((double)r1, (double)r1, r2);
+        r2 = fma((double)rb, (double)rb, r2);
+
+        const float rQ = __fmul_rn(__fmul_rn(Q, S), rden);   // 1/Q
+        const float nrS = -__fmul_rn(QQ, rden);              // -1/S
+        const float m4 = __fmul_rn(-4.0f, rQ);
+        const float2 t10 = mul2(mul2(s01, f2(s2)), t10c);
+        const float t2 = __fmul_rn(__fmul_rn(s01.x, s01.y), t2c);
+        const float2 d01 = add2(make_float2(x2.x, x2.y), make_float2(y2v.x, y2v.y));
+        const float2 d23 = add2(make_float2(x2.z, x2.w), make_float2(y2v.z, y2v.w));
+        const float d4 = __fadd_rn(x1.w, y1v.w);
+        const float2 A = mul2(f2(ks), fma2(rs, fma2(mul2(uv4, q01), f2(rQ), f2(-1.0f)), mul2(d01, f2(nrS))));
+        const float2 dq = fma2(om2, f2(t2), fma2(om0, f2(t10.y), mul2(om1, f2(t10.x))));
+        const float2 B = mul2(f2(ks), fma2(f2(m4), dq, mul2(d23, f2(nrS))));
+        const float V6 = __fmul_rn(ks, __fmaf_rn(m4, t2, __fmul_rn(d4, nrS)));
+        const float2 Cv = make_float2(V6, ks_on);
+
+        const float P = __fmaf_rn(sp1, sp1, __fmul_rn(sp2, sp2));
+        const float2 hr1 = make_float2(h1, r1), hr2 = make_float2(h2, rb);
+        const float2 XR = fma2(f2(sp1), hr1, mul2(f2(sp2), hr2));
+        const float2 ZU = fma2(f2(h1), hr1, mul2(f2(h2), hr2));
+        const float X = __fmul_rn(kd_on, XR.x);
+        const float2 PA = mul2(f2(P), A), PB = mul2(f2(P), B);
+        const float P6 = __fmul_rn(P, V6), P2 = __fmul_rn(P, ks_on);
+        a.h0A = fma2(f2(PA.x), A, a.h0A);
+        a.h0B = fma2(f2(PA.x), B, a.h0B);
+        a.h0C = fma2(f2(PA.x), Cv, a.h0C);
+        a.h11 = __fmaf_rn(PA.y, A.y, a.h11);
+        a.h1B = fma2(f2(PA.y), B, a.h1B);
+        a.h1C = fma2(f2(PA.y), Cv, a.h1C);
+        a.h2B = fma2(f2(P2), B, a.h2B);
+        a.h2C = fma2(f2(P2), Cv, a.h2C);
+        a.h4B = fma2(f2(PB.x), B, a.h4B);
+        a.h45_6 = fma2(PB, f2(V6), a.h45_6);
+        a.h55 = __fmaf_rn(PB.y, B.y, a.h55);
+        a.h66 = __fmaf_rn(P6, V6, a.h66);
+        a.xA = fma2(f2(X), A, a.xA);
+        a.xB = fma2(f2(X), B, a.xB);
+        a.xC = fma2(f2(X), Cv, a.xC);
+        a.rA = fma2(f2(XR.y), A, a.rA);
+        a.rB = fma2(f2(XR.y), B, a.rB);
+        a.rC = fma2(f2(XR.y), Cv, a.rC);
+        a.zu = fma2(f2(kd_on), ZU, a.zu);   // (kd_on is 0 or 1: the product is exact)
+    }
+};
+
 // ------------------------------------------------------------------------------
 // packed pair evaluation: two unordered pairs per lane, one in each half of the
 // sm_100 paired FP32 instructions (add/mul/fma .f32x2), for the luminance fit
 // without a Fresnel factor.  Arithmetic per pair as in sym_pair; the two halves
 // accumulate separately and are added once at the end of the pass.
 // ------------------------------------------------------------------------------
-
-__device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b)
-{
-    float2 r;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "sub.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
 
 // Per-pass constants of sym_pair in paired form (both halves equal), with the
 // products that do not depend on the pair folded in.
@@ -1057,16 +1215,66 @@ __device__ __forceinline__ void pair_step(const float* tab, const PassConst& c, 
     }
 }
 
+// pair_step of the luminance fit without a Fresnel factor.
+template <int NW, bool kAllUp, bool kGuard>
+__device__ __forceinline__ void lum_step(const LumPass& pass, const float* tab, const float* fs, uint32_t L, uint32_t Lp,
+                                         uint32_t nd, uint32_t total, uint32_t sa, uint32_t sd, uint32_t& f, uint32_t& a,
+                                         uint32_t& d, LumSums& sums, double& r2)
+{
+    const bool valid = !kGuard || (f < total && !(2u * d == L && a >= (L >> 1)));
+    uint32_t b = a + d;
+    b = b >= L ? b - L : b;
+    const uint32_t ia = valid ? a : 0u, ib = valid ? b : 0u;
+    const float4* core0 = reinterpret_cast<const float4*>(tab);
+    const float4 x0 = core0[ia], x1 = core0[Lp + ia], x2 = core0[2 * Lp + ia];
+    const float4 y0 = core0[ib], y1v = core0[Lp + ib], y2v = core0[2 * Lp + ib];
+    const bool two = valid && d != 0u;
+    const float y1 = valid ? fs[ia * L + ib] : 0.0f;
+    const float y2 = two ? fs[ib * L + ia] : 0.0f;
+    pass.add<kAllUp, kGuard>(x0, x1, x2, y0, y1v, y2v, y1, y2, kGuard ? (valid ? 1.0f : 0.0f) : 1.0f, two ? 1.0f : 0.0f,
+                             sums, r2);
+    f += 32u * NW;
+    a += sa;
+    d += sd;
+    if(d >= nd)
+    {
+        d -= nd;
+        ++a;
+    }
+}
+
+// A worker warp's sums over its lanes to red[wwarp][0..kAcc) and redd[wwarp].
+template <int kAcc>
+__device__ __forceinline__ void store_partials(float* acc, double r2, float* red, double* redd, uint32_t wwarp,
+                                               uint32_t lane)
+{
+    static_assert(kAcc >= 32, "reduction layout: 32 reduce-scattered sums + the rest");
+    r2 = warp_sum(r2);
+    float rest[kAcc - 32];
+#pragma unroll
+    for(int i = 32; i < kAcc; ++i)
+        rest[i - 32] = warp_sum(acc[i]);
+    reduce_scatter32(acc, lane);
+    red[wwarp * kAcc + lane] = acc[0];
+    if(lane == 0)
+    {
+#pragma unroll
+        for(int i = 32; i < kAcc; ++i)
+            red[wwarp * kAcc + i] = rest[i - 32];
+        redd[wwarp] = r2;
+    }
+}
+
 // One worker warp's share of a pass over the pairs of a slot (unordered pairs
 // wtid, wtid + 32 NW, ...).  Writes the warp's partial sums: J^T J and J^T r
 // to red[wwarp][0..34] and r^2 to redd[wwarp].  Every lane runs the same
 // number of steps; for odd L only the last one needs the guard.
-template <class M, int NW, bool kFresnel, bool kAllUp>
+// kPaired: the luminance fit without a Fresnel factor steps by LumPass::add.
+template <class M, int NW, bool kFresnel, bool kAllUp, bool kPaired = false>
 __device__ void worker_pass(const float* tab, const PassConst& c, const typename M::Slab* slab, uint32_t L,
                             float refr, float* red, double* redd, uint32_t wwarp, uint32_t lane)
 {
     constexpr int kAcc = M::kAcc;
-    static_assert(kAcc >= 32, "reduction layout: 32 reduce-scattered sums + the rest");
     constexpr uint32_t kStride = 32u * NW;
     const uint32_t half = L >> 1, nd = half + 1, Lp = pad4(L);
     const uint32_t total = L * nd;
@@ -1078,30 +1286,29 @@ __device__ void worker_pass(const float* tab, const PassConst& c, const typename
 
     double r2 = 0.0;
     float acc[kAcc];
-#pragma unroll
-    for(int i = 0; i < kAcc; ++i)
-        acc[i] = 0.0f;
-
-    for(uint32_t it = 0; it < full; ++it)
-        pair_step<M, NW, kFresnel, kAllUp, false>(tab, c, slab, L, Lp, nd, total, sa, sd, refr, f, a, d, acc, r2);
-    for(uint32_t it = full; it < iters; ++it)
-        pair_step<M, NW, kFresnel, kAllUp, true>(tab, c, slab, L, Lp, nd, total, sa, sd, refr, f, a, d, acc, r2);
-
-    r2 = warp_sum(r2);
+    if constexpr(!M::kRgb && !kFresnel && kPaired)
     {
-        float rest[kAcc - 32];
-#pragma unroll
-        for(int i = 32; i < kAcc; ++i)
-            rest[i - 32] = warp_sum(acc[i]);
-        reduce_scatter32(acc, lane);
-        red[wwarp * kAcc + lane] = acc[0];
-        if(lane == 0)
-#pragma unroll
-            for(int i = 32; i < kAcc; ++i)
-                red[wwarp * kAcc + i] = rest[i - 32];
+        const LumPass pass(c);
+        LumSums sums;
+        sums.clear();
+        const float* fs = reinterpret_cast<const float*>(slab);
+        for(uint32_t it = 0; it < full; ++it)
+            lum_step<NW, kAllUp, false>(pass, tab, fs, L, Lp, nd, total, sa, sd, f, a, d, sums, r2);
+        for(uint32_t it = full; it < iters; ++it)
+            lum_step<NW, kAllUp, true>(pass, tab, fs, L, Lp, nd, total, sa, sd, f, a, d, sums, r2);
+        sums.unpack(acc);
     }
-    if(lane == 0)
-        redd[wwarp] = r2;
+    else
+    {
+#pragma unroll
+        for(int i = 0; i < kAcc; ++i)
+            acc[i] = 0.0f;
+        for(uint32_t it = 0; it < full; ++it)
+            pair_step<M, NW, kFresnel, kAllUp, false>(tab, c, slab, L, Lp, nd, total, sa, sd, refr, f, a, d, acc, r2);
+        for(uint32_t it = full; it < iters; ++it)
+            pair_step<M, NW, kFresnel, kAllUp, true>(tab, c, slab, L, Lp, nd, total, sa, sd, refr, f, a, d, acc, r2);
+    }
+    store_partials<kAcc>(acc, r2, red, redd, wwarp, lane);
 }
 
 // The row fit of LeastSquaresFitSGGX's LSF_OPTION_FIT_TOP
@@ -1132,20 +1339,7 @@ __device__ void worker_pass_row(const float* tab, const PassConst& c, const floa
         const Entry eb = load_entry(tab, Lp, valid ? b : 0u);
         sym_pair<kFresnel, kAllUp>(c, ea, eb, refr, valid ? row[b] : 0.0f, 0.0f, valid ? 1.0f : 0.0f, 0.0f, acc, r2);
     }
-    r2 = warp_sum(r2);
-    float rest[kAcc - 32];
-#pragma unroll
-    for(int i = 32; i < kAcc; ++i)
-        rest[i - 32] = warp_sum(acc[i]);
-    reduce_scatter32(acc, lane);
-    red[wwarp * kAcc + lane] = acc[0];
-    if(lane == 0)
-    {
-#pragma unroll
-        for(int i = 32; i < kAcc; ++i)
-            red[wwarp * kAcc + i] = rest[i - 32];
-        redd[wwarp] = r2;
-    }
+    store_partials<kAcc>(acc, r2, red, redd, wwarp, lane);
 }
 
 // Advances an unordered pair (f, a, d) by one worker stride (sa, sd): f += 32 NW.
@@ -1236,21 +1430,7 @@ __device__ void worker_pass2(const float* tab, const PassConst& c1, const float*
 #pragma unroll
     for(int i = 0; i < kAcc; ++i)
         acc[i] = acc2[i].x + acc2[i].y;
-    r2 = warp_sum(r2);
-    {
-        float rest[kAcc - 32];
-#pragma unroll
-        for(int i = 32; i < kAcc; ++i)
-            rest[i - 32] = warp_sum(acc[i]);
-        reduce_scatter32(acc, lane);
-        red[wwarp * kAcc + lane] = acc[0];
-        if(lane == 0)
-#pragma unroll
-            for(int i = 32; i < kAcc; ++i)
-                red[wwarp * kAcc + i] = rest[i - 32];
-    }
-    if(lane == 0)
-        redd[wwarp] = r2;
+    store_partials<kAcc>(acc, r2, red, redd, wwarp, lane);
 }
 
 // worker_pass with J^T J on the tensor cores.  Each step every lane stages the
@@ -1495,12 +1675,12 @@ __device__ void write_texel(const LmArgs& args, LmState<M::P>& st, uint32_t t, d
 }
 }
 
-// Control thread: takes the next texel for slot `sl` and starts its slab copy
-// (the slab is no longer read: the workers finished the slot's last pass).
+// Control thread: puts texel c of the launch (none past its texels) into slot
+// `sl` and starts its slab copy (the slab is no longer read: the workers
+// finished the slot's last pass).
 template <class M>
-__device__ __forceinline__ void slot_fetch(const LmArgs& args, Slot<M>& sl, void* slab)
+__device__ __forceinline__ void slot_take(const LmArgs& args, Slot<M>& sl, void* slab, uint32_t c)
 {
-    const uint32_t c = sl.dead ? kNoTexel : atomicAdd(args.work_counter, 1u);
     if(c < args.texels)
     {
         const uint32_t t = args.texel_base + c;
@@ -1529,6 +1709,13 @@ __device__ __forceinline__ void slot_fetch(const LmArgs& args, Slot<M>& sl, void
         sl.loading = 0;
     }
     sl.cmd = kSlotIdle;
+}
+
+// The next texel of the launch's counter.
+template <class M>
+__device__ __forceinline__ void slot_fetch(const LmArgs& args, Slot<M>& sl, void* slab)
+{
+    slot_take(args, sl, slab, sl.dead ? kNoTexel : args.counter_base + atomicAdd(args.work_counter, 1u));
 }
 
 // Control thread: the slot's slab has arrived; set up the fit of its texel.
@@ -1660,6 +1847,68 @@ __device__ void expand_sums(const double* sums, const float* pf, double* hg)
 }
 }
 
+// Lane 0, after a slot's pass (its sums in sl.sums): the LM step.  True when
+// sl.pf holds the next point to evaluate, of this texel or, its outputs written,
+// of the next one the slot took; false when the slot has no texel left.
+template <class M>
+__device__ __forceinline__ bool slot_step(const LmArgs& args, Slot<M>& sl, void* slab)
+{
+    LmState<M::P>& st = sl.st;
+    int next = kCmdDone;
+    // Every pass evaluates J^T J and J^T r with r^2: at a trial point
+    // the Jacobian of an accepted step is then already at hand, so
+    // the separate Jacobian evaluation of fitting.hh:612-616 at the
+    // same point is not repeated (same arithmetic, same result).
+    constexpr int kH = M::P * (M::P + 1) / 2;
+    expand_sums<M>(sl.sums, sl.pf, sl.hg);
+    if(sl.first)
+    {
+        sl.first = 0;
+        st.njac = 1;
+        st.S = sl.sums[M::kAcc];
+#pragma unroll
+        for(int i = 0; i < M::P; ++i)
+            st.g[i] = (st.fixed & (1u << i)) ? 0.0 : -sl.hg[kH + i];
+#pragma unroll
+        for(int i = 0; i < kH; ++i)
+            st.H[i] = sl.hg[i];
+        lm_reset_damping(st);
+        if(!isfinite(st.S))
+            st.status |= SVF_TEXEL_NONFINITE;
+        next = kCmdContinue;
+    }
+    else
+    {
+        next = lm_after_trial<M>(st, args.cfg, sl.sums[M::kAcc], sl.npairs);
+        if(next == kCmdJacobian)
+            next = lm_after_jacobian(st, args.cfg, sl.hg, sl.npairs);
+    }
+    if(next == kCmdContinue)
+        next = lm_next<M>(st, args.cfg, sl.npairs);
+    if(next == kCmdTrial)
+    {
+        if constexpr(M::kRgb)
+        {
+            for(int i = 0; i < M::B; ++i)
+                sl.pf[i] = (float)st.pt[i];
+            for(int i = 0; i < 4; ++i)
+                sl.pf[M::B + i] = (float)st.qt[i];
+        }
+        else
+#pragma unroll
+            for(int i = 0; i < M::P; ++i)
+                sl.pf[i] = (float)st.pt[i];
+        sl.cmd = kSlotPass;
+        return true;
+    }
+    write_texel<M>(args, st, sl.texel, sl.npairs);
+    slot_fetch(args, sl, slab);
+    // the next texel starts at once (its slab copy is short next to the passes
+    // of the other slots, which run meanwhile) rather than after a round with
+    // the slot idle
+    return sl.loading && slot_start(args, sl);
+}
+
 // Resident CTAs per SM the register budget is sized for.
 // Resident CTAs the register budget is sized for (128 registers a thread at
 // 128 and 160 threads).
@@ -1788,67 +2037,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), kPass == kPassPacked ? 1 : min_
         bool build = false, exit_now = false;
         if(lane == 0)
         {
-            LmState<M::P>& st = sl.st;
-            int next = kCmdDone;
             if(done_cmd == kSlotPass)
-            {
-                // Every pass evaluates J^T J and J^T r with r^2: at a trial point
-                // the Jacobian of an accepted step is then already at hand, so
-                // the separate Jacobian evaluation of fitting.hh:612-616 at the
-                // same point is not repeated (same arithmetic, same result).
-                constexpr int kH = M::P * (M::P + 1) / 2;
-                expand_sums<M>(sl.sums, sl.pf, sl.hg);
-                if(sl.first)
-                {
-                    sl.first = 0;
-                    st.njac = 1;
-                    st.S = sl.sums[M::kAcc];
-#pragma unroll
-                    for(int i = 0; i < M::P; ++i)
-                        st.g[i] = (st.fixed & (1u << i)) ? 0.0 : -sl.hg[kH + i];
-#pragma unroll
-                    for(int i = 0; i < kH; ++i)
-                        st.H[i] = sl.hg[i];
-                    lm_reset_damping(st);
-                    if(!isfinite(st.S))
-                        st.status |= SVF_TEXEL_NONFINITE;
-                    next = kCmdContinue;
-                }
-                else
-                {
-                    next = lm_after_trial<M>(st, args.cfg, sl.sums[M::kAcc], sl.npairs);
-                    if(next == kCmdJacobian)
-                        next = lm_after_jacobian(st, args.cfg, sl.hg, sl.npairs);
-                }
-                if(next == kCmdContinue)
-                    next = lm_next<M>(st, args.cfg, sl.npairs);
-                if(next == kCmdTrial)
-                {
-                    if constexpr(M::kRgb)
-                    {
-                        for(int i = 0; i < M::B; ++i)
-                            sl.pf[i] = (float)st.pt[i];
-                        for(int i = 0; i < 4; ++i)
-                            sl.pf[M::B + i] = (float)st.qt[i];
-                    }
-                    else
-#pragma unroll
-                        for(int i = 0; i < M::P; ++i)
-                            sl.pf[i] = (float)st.pt[i];
-                    sl.cmd = kSlotPass;
-                    build = true;
-                }
-                else
-                {
-                    write_texel<M>(args, st, sl.texel, sl.npairs);
-                    slot_fetch(args, sl, slab_of(s));
-                    // the next texel starts in this visit (its slab copy is short
-                    // next to the other slots' passes, which the workers run
-                    // meanwhile) rather than after a round with the slot idle
-                    if(sl.loading)
-                        build = slot_start(args, sl);
-                }
-            }
+                build = slot_step<M>(args, sl, slab_of(s));
             else if(sl.loading)
             {
                 // the slab was requested during an earlier visit
@@ -1890,14 +2080,276 @@ __global__ void __launch_bounds__(32 * (NW + 1), kPass == kPassPacked ? 1 : min_
     }
 }
 
+// ------------------------------------------------------------------------------
+// the pooled persistent kernel (the plain pair pass)
+// ------------------------------------------------------------------------------
+
+// One CTA of 8 warps per SM over S texel slots, every warp doing whatever
+// is ready: a *share* of a slot's pass (the pairs wtid = 32 share + lane, + 32 NW,
+// ..; NW shares a pass), or, for the warp that finished a slot's last share, the
+// slot's LM step (lane 0, FP64), the next direction table (32 lanes) and the
+// texel's outputs.  A share's sums do not depend on the warp that computed them
+// and the shares are added in share order, so a texel's result depends on NW
+// alone.
+//
+// Where it is used: the RGB fit, and luminance passes of 7 shares (layouts whose
+// slabs leave room for two texels an SM).  The warp-specialised kernel gives those
+// one CTA of 7 workers or two, which wait for their control warp (RGB: its FP64 step
+// on 11 parameters takes longer than a pass) or for the slowest of them, two
+// workers to a scheduler and one beside the control warp.  Measured against it:
+// RGB LM of 173 x 173 ring-81 texels 25.4 -> 18.9 ms, 97 x 97 Fibonacci-151 texels
+// 8.88 -> 8.17 ms.  On ring-81 luminance slabs, 7 slots of 4 shares here and three
+// CTAs of 4 workers there, both keep the SM's FP32 pipe at what its operand reads
+// allow (400 x 400: 46.3 and 46.8 ms), and the shorter launches end later here
+// (150 x 150: 7.6 and 7.4 ms), so those stay where they were.
+//
+// Slot hand-over (all in shared memory): the table, constants and slab of a slot
+// are complete, then its sequence number, then a fence, then its shares' bits in
+// `open`; a share is claimed by clearing its bit.
+// Order: the slot published first, so that passes complete one after the other
+// and a texel with many iterations waits no longer than the others (dealing the
+// warps over all slots leaves too many passes waiting for their last share: 50.1
+// against 45.3 ms for 400 x 400 ring-81 texels).  Of that slot a warp takes a
+// share of its scheduler, u = (warp - s) mod 4 (the SM deals a CTA's warps to its
+// four schedulers in turn), and another one only on a second look, so that the
+// shares of the few texels a launch ends with spread over the schedulers.
+// Two warps a scheduler, with all the registers they ask for (luminance 180, RGB
+// 255): a pass's steps are bound by the FP32 pipe's operand reads (luminance: 225
+// cycles a step and scheduler with two warps on it, 200 with four), so that more
+// warps at 128 registers gain little and lose by what they spill (RGB, 173 x 173:
+// 23.0 ms with 16 warps, 18.9 with 8; Fibonacci-151, 97 x 97: 10.4 and 8.2 ms).
+constexpr int kPoolWarps = 8, kPoolMaxSlots = 16;
+
+struct PoolCtl
+{
+    uint32_t sequence;   // passes published
+    uint32_t live;       // slots with a texel
+    uint32_t progress;   // shares done (the bound of an idle warp's wait counts waits without progress)
+    uint32_t abort;      // an idle wait ran out: every warp leaves
+    uint32_t epoch;      // phase of `wake`
+    uint64_t wake;       // mbarrier, one phase per event an idle warp waits for: shares published, a slot done
+    uint32_t open[kPoolMaxSlots];     // a slot's unclaimed shares
+    uint32_t number[kPoolMaxSlots];   // and its pass's number among the CTA's passes
+};
+
+constexpr uint64_t kPoolIdleNs = 2000000000ull;   // an idle warp's wait without any progress in the CTA: 2 s
+constexpr uint32_t kPoolNapNs = 500;              // and the time between its looks
+
+template <class M>
+__host__ __device__ constexpr size_t pool_slot_bytes(int nw, uint32_t L, uint64_t stride)
+{
+    // SlotSmem<nw, M>::bytes and the slot's control state
+    return SlotSmem<1, M>::slab_bytes(stride) + SlotSmem<1, M>::tab_bytes(L) +
+           ((sizeof(float) * nw * M::kAcc + sizeof(double) * nw + 127) & ~size_t(127)) +
+           ((sizeof(Slot<M>) + 127) & ~size_t(127));
+}
+
+template <class M, int NW, bool kFresnel, bool kAllUp>
+__global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args, uint32_t S)
+{
+    using SM = SlotSmem<NW, M>;
+    using SlabT = typename M::Slab;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ PoolCtl ctl;
+    volatile PoolCtl* vctl = &ctl;
+
+    const uint32_t per_slot = (uint32_t)pool_slot_bytes<M>(NW, args.L, args.lum_stride);
+    const uint32_t tab_at = (uint32_t)SM::slab_bytes(args.lum_stride);
+    const uint32_t red_at = tab_at + (uint32_t)SM::tab_bytes(args.L);
+    const uint32_t slot_at = red_at + (uint32_t)SM::red_bytes();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    auto slot_of = [&](uint32_t s) -> Slot<M>& { return *reinterpret_cast<Slot<M>*>(smem_raw + s * per_slot + slot_at); };
+
+    // lane 0: ends the phase idle warps wait for (after what they look for is in place)
+    auto wake_idle = [&]() {
+        __threadfence_block();
+        atomicAdd(&ctl.epoch, 1u);
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&ctl.wake)) : "memory");
+    };
+    // all lanes: slot s's shares are there to claim (build), or it has no texel left
+    auto publish = [&](uint32_t s, bool build) {
+        __syncwarp();
+        if(lane == 0)
+        {
+            if(build)
+            {
+                ctl.number[s] = atomicAdd(&ctl.sequence, 1u);
+                __threadfence_block();
+                atomicExch(&ctl.open[s], (1u << NW) - 1u);
+            }
+            else
+                atomicSub(&ctl.live, 1u);
+            wake_idle();
+        }
+    };
+
+    if(threadIdx.x == 0)
+    {
+        ctl.sequence = 0;
+        ctl.live = S;
+        ctl.progress = 0;
+        ctl.abort = 0;
+        ctl.epoch = 0;
+        mbar_init(&ctl.wake, 1);
+    }
+    if(threadIdx.x < S)
+        ctl.open[threadIdx.x] = 0;   // (every warp looks at every slot from here on)
+    __syncthreads();
+    for(uint32_t s = warp; s < S; s += warps)
+    {
+        Slot<M>& sl = slot_of(s);
+        unsigned char* base = smem_raw + s * per_slot;
+        bool build = false;
+        if(lane == 0)
+        {
+            mbar_init(&sl.bar, 1);
+            sl.parity = 0;
+            sl.dead = 0;
+            sl.drain = 0;
+            sl.arrived = 0;
+            // the first texels go round the CTAs, so that a launch of few texels
+            // spreads over the SMs
+            slot_take(args, sl, base, s * gridDim.x + blockIdx.x);
+            build = sl.loading && slot_start(args, sl);
+        }
+        __syncwarp();
+        build = __shfl_sync(0xffffffffu, build, 0);
+        if(build)
+            build_table<M>(reinterpret_cast<float*>(base + tab_at), sl.geo, sl.L, sl.pf, &sl.pc, lane);
+        publish(s, build);
+    }
+
+    // lane s watches slot s
+    static_assert(kPoolMaxSlots <= 32, "a lane per slot");
+    uint32_t seen = 0;
+    uint64_t idle_since = 0;   // 0: not idle
+    bool second = false;   // this is a second look
+    for(;;)
+    {
+        const uint32_t epoch = vctl->epoch;   // (read before `open`: a later publication ends a phase from here on)
+        const bool leave = vctl->live == 0 || vctl->abort;
+        const uint32_t open = lane < S ? vctl->open[lane] : 0u;
+        const uint32_t first = __reduce_min_sync(0xffffffffu, open ? (vctl->number[lane] << 5) | lane : 0xffffffffu);
+        if(first != 0xffffffffu)
+        {
+            // claim a share of that slot
+            const uint32_t s = first & 31u;
+            Slot<M>& sl = slot_of(s);
+            uint32_t share = NW;
+            if(lane == s)
+            {
+                const uint32_t own = open & (0x11111111u << ((warp - s) & 3u));
+                const uint32_t pick = own ? own : (second ? open : 0u);
+                const uint32_t u = (uint32_t)__ffs((int)pick) - 1u;
+                if(pick && (atomicAnd(&ctl.open[s], ~(1u << u)) & (1u << u)))
+                    share = u;
+                __threadfence_block();
+            }
+            __syncwarp();   // orders the claim before the other lanes' reads of the slot
+            share = __shfl_sync(0xffffffffu, share, s);
+            second = share == (uint32_t)NW;
+            if(second)
+                continue;   // (another scheduler's share, or another warp was faster)
+            idle_since = 0;
+            unsigned char* base = smem_raw + s * per_slot;
+            float* tab = reinterpret_cast<float*>(base + tab_at);
+            double* redd = reinterpret_cast<double*>(base + red_at);
+            float* red = reinterpret_cast<float*>(redd + NW);
+            worker_pass<M, NW, kFresnel, kAllUp, true>(tab, sl.pc, reinterpret_cast<const SlabT*>(base), sl.L,
+                                                       args.cfg.fresnel, red, redd, share, lane);
+            __syncwarp();
+            uint32_t prior = 0;
+            if(lane == 0)
+            {
+                __threadfence_block();   // release this share's sums
+                prior = atomicAdd(&sl.arrived, 1u);
+                atomicAdd(&ctl.progress, 1u);
+                __threadfence_block();   // acquire the other shares' sums
+            }
+            prior = __shfl_sync(0xffffffffu, prior, 0);
+            if(prior != (uint32_t)NW - 1u)
+                continue;
+            // the pass is complete: sum the shares, step, tabulate the next point
+            __syncwarp();
+            sum_partials<NW, M::kAcc>(red, redd, sl.sums, lane);
+            __syncwarp();
+            bool build = false;
+            if(lane == 0)
+            {
+                sl.arrived = 0;
+                build = slot_step<M>(args, sl, base);
+            }
+            __syncwarp();   // orders lane 0's slot updates before the other lanes read them
+            build = __shfl_sync(0xffffffffu, build, 0);
+            if(build)
+                build_table<M>(tab, sl.geo, sl.L, sl.pf, &sl.pc, lane);
+            publish(s, build);
+            continue;
+        }
+        if(__any_sync(0xffffffffu, leave))
+            break;
+        const uint32_t p = __shfl_sync(0xffffffffu, vctl->progress, 0);
+        const uint64_t now = __shfl_sync(0xffffffffu, global_ns(), 0);
+        if(p != seen || !idle_since)
+        {
+            seen = p;
+            idle_since = now;
+        }
+        else if(now - idle_since > kPoolIdleNs)
+        {
+            if(lane == 0)
+            {
+                vctl->abort = 1;
+                atomicOr(args.error_flag, 1u);
+            }
+            break;
+        }
+        // suspended until the phase ends, kPoolNapNs at most (a phase of the same
+        // parity may have come and gone in between)
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1, %2;\n\t}" ::"r"(smem_addr(&ctl.wake)),
+                     "r"(epoch & 1u), "r"(kPoolNapNs)
+                     : "memory");
+    }
+    // a slab copy whose wait expired may still be in flight: wait for it
+    // (bounded again) before the CTA's shared memory is released
+    __syncthreads();
+    if(threadIdx.x == 0)
+        for(uint32_t s = 0; s < S; ++s)
+            if(slot_of(s).drain)
+                mbar_wait(&slot_of(s).bar, slot_of(s).parity, args.wait_spins);
+}
+
 using KernelFn = void (*)(LmArgs);
 
-template <class M, int NW, int S>
-KernelFn pick(bool fresnel, bool all_up)
+using PoolFn = void (*)(LmArgs, uint32_t);
+
+template <class M, int NW>
+PoolFn pick_pool(bool fresnel, bool all_up)
 {
     if(fresnel)
-        return all_up ? lm_fit_kernel<M, NW, S, true, true, kPassPlain> : lm_fit_kernel<M, NW, S, true, false, kPassPlain>;
-    return all_up ? lm_fit_kernel<M, NW, S, false, true, kPassPlain> : lm_fit_kernel<M, NW, S, false, false, kPassPlain>;
+        return all_up ? lm_pool_kernel<M, NW, true, true> : lm_pool_kernel<M, NW, true, false>;
+    return all_up ? lm_pool_kernel<M, NW, false, true> : lm_pool_kernel<M, NW, false, false>;
+}
+
+// The pooled kernel of a configuration (its worker count NW is the number of
+// shares of a pass), or null.
+template <class M>
+PoolFn pool_for_model(LmKernelChoice c, bool fresnel, bool all_up)
+{
+    if(c.pass != kPassPlain && !(M::kRgb || (fresnel && c.pass != kPassRow)))
+        return nullptr;
+    // (a packed or tensor-core choice runs the plain pass where those do not apply)
+    if(c.threads == 256)
+        return pick_pool<M, 7>(fresnel, all_up);
+    if constexpr(M::kRgb)
+    {
+        if(c.threads == 128)
+            return pick_pool<M, 3>(fresnel, all_up);
+        if(c.threads == 160)
+            return pick_pool<M, 4>(fresnel, all_up);
+    }
+    return nullptr;
 }
 
 // The packed and tensor-core instances (luminance, no Fresnel factor).
@@ -1907,62 +2359,72 @@ KernelFn pick_pass(bool all_up)
     return all_up ? lm_fit_kernel<LumModel, NW, S, false, true, kPass> : lm_fit_kernel<LumModel, NW, S, false, false, kPass>;
 }
 
-template <class M>
-KernelFn kernel_for_model(LmKernelChoice c, bool fresnel, bool all_up)
+// The luminance kernels with a plain pass of 3 or 4 workers.
+template <int NW, int S>
+KernelFn pick(bool fresnel, bool all_up)
 {
-    if constexpr(!M::kRgb)
-        if(c.pass == kPassRow)
-        {
-            // a row slab is L floats: one configuration serves every layout
-            if(c.threads != 256 || c.slots != 2)
-                return nullptr;
-            if(fresnel)
-                return all_up ? lm_fit_kernel<LumModel, 7, 2, true, true, kPassRow>
-                              : lm_fit_kernel<LumModel, 7, 2, true, false, kPassRow>;
-            return all_up ? lm_fit_kernel<LumModel, 7, 2, false, true, kPassRow>
-                          : lm_fit_kernel<LumModel, 7, 2, false, false, kPassRow>;
-        }
-        else if(c.pass == kPassPacked && !fresnel)
-        {
-            if(c.threads == 256 && c.slots == 3)
-                return pick_pass<7, 3, kPassPacked>(all_up);
-            if(c.threads == 256 && c.slots == 4)
-                return pick_pass<7, 4, kPassPacked>(all_up);
-            if(c.threads == 128 && c.slots == 3)
-                return pick_pass<3, 3, kPassPacked>(all_up);
+    if(fresnel)
+        return all_up ? lm_fit_kernel<LumModel, NW, S, true, true, kPassPlain>
+                      : lm_fit_kernel<LumModel, NW, S, true, false, kPassPlain>;
+    return all_up ? lm_fit_kernel<LumModel, NW, S, false, true, kPassPlain>
+                  : lm_fit_kernel<LumModel, NW, S, false, false, kPassPlain>;
+}
+
+// The warp-specialised kernel of a luminance configuration, or null.
+KernelFn kernel_for(LmKernelChoice c, bool fresnel, bool all_up)
+{
+    if(c.pass == kPassRow)
+    {
+        // a row slab is L floats: one configuration serves every layout
+        if(c.threads != 256 || c.slots != 2)
             return nullptr;
-        }
-        else if(c.pass == kPassTc && !fresnel)
-        {
-            if(c.threads == 256 && c.slots == 2)
-                return pick_pass<7, 2, kPassTc>(all_up);
-            if(c.threads == 128 && c.slots == 3)
-                return pick_pass<3, 3, kPassTc>(all_up);
-            return nullptr;
-        }
+        if(fresnel)
+            return all_up ? lm_fit_kernel<LumModel, 7, 2, true, true, kPassRow>
+                          : lm_fit_kernel<LumModel, 7, 2, true, false, kPassRow>;
+        return all_up ? lm_fit_kernel<LumModel, 7, 2, false, true, kPassRow>
+                      : lm_fit_kernel<LumModel, 7, 2, false, false, kPassRow>;
+    }
+    if(c.pass == kPassPacked && !fresnel)
+    {
+        if(c.threads == 256 && c.slots == 3)
+            return pick_pass<7, 3, kPassPacked>(all_up);
+        if(c.threads == 256 && c.slots == 4)
+            return pick_pass<7, 4, kPassPacked>(all_up);
+        if(c.threads == 128 && c.slots == 3)
+            return pick_pass<3, 3, kPassPacked>(all_up);
+        return nullptr;
+    }
+    if(c.pass == kPassTc && !fresnel)
+    {
+        if(c.threads == 256 && c.slots == 2)
+            return pick_pass<7, 2, kPassTc>(all_up);
+        if(c.threads == 128 && c.slots == 3)
+            return pick_pass<3, 3, kPassTc>(all_up);
+        return nullptr;
+    }
     // (a packed or tensor-core choice runs the plain pass where those do not apply)
-    if(c.threads == 256 && c.slots == 2)
-        return pick<M, 7, 2>(fresnel, all_up);
-    if(c.threads == 256 && c.slots == 3)
-        return pick<M, 7, 3>(fresnel, all_up);
-    if(c.threads == 256 && c.slots == 4)
-        return pick<M, 7, 4>(fresnel, all_up);
     if(c.threads == 128 && c.slots == 2)
-        return pick<M, 3, 2>(fresnel, all_up);
+        return pick<3, 2>(fresnel, all_up);
     if(c.threads == 128 && c.slots == 3)
-        return pick<M, 3, 3>(fresnel, all_up);
+        return pick<3, 3>(fresnel, all_up);
     if(c.threads == 160 && c.slots == 2)
-        return pick<M, 4, 2>(fresnel, all_up);
+        return pick<4, 2>(fresnel, all_up);
     if(c.threads == 160 && c.slots == 3)
-        return pick<M, 4, 3>(fresnel, all_up);
-    if(c.threads == 256 && c.slots == 1)   // the largest slabs: one texel per CTA, no overlap
-        return pick<M, 7, 1>(fresnel, all_up);
+        return pick<4, 3>(fresnel, all_up);
     return nullptr;
 }
 
-KernelFn kernel_for(LmKernelChoice c, bool fresnel, bool all_up, bool rgb)
+PoolFn pool_for(LmKernelChoice c, bool fresnel, bool all_up, bool rgb)
 {
-    return rgb ? kernel_for_model<RgbModel>(c, fresnel, all_up) : kernel_for_model<LumModel>(c, fresnel, all_up);
+    return rgb ? pool_for_model<RgbModel>(c, fresnel, all_up) : pool_for_model<LumModel>(c, fresnel, all_up);
+}
+
+// Slots of slabs of this size that one CTA's shared memory holds.
+uint32_t pool_slots(int nw, uint32_t L, uint64_t stride, bool rgb)
+{
+    const size_t per = rgb ? pool_slot_bytes<RgbModel>(nw, L, stride) : pool_slot_bytes<LumModel>(nw, L, stride);
+    constexpr size_t kMaxDynamic = 227u * 1024u - 256u;   // (the static part takes PoolCtl)
+    return (uint32_t)std::min<size_t>(kPoolMaxSlots, kMaxDynamic / per);
 }
 
 } // namespace
@@ -1977,6 +2439,9 @@ LmKernelChoice lm_default_choice(uint32_t L, uint64_t lum_stride, bool rgb)
     // 128 threads x 2 slots (3 CTAs, 6 texels per SM) 52.2 ms, 256 x 2 54.7,
     // 256 x 3 55.9, 128 x 3 57.7; Fibonacci-151 slabs, 589824 texels --
     // 256 x 2 (1 CTA) 564 ms, 256 x 1 (2 CTAs) 595, 128 x 2 773.
+    // A pass is summed in threads / 32 - 1 parts, so the choice also fixes the order
+    // of a texel's sums; the configurations that run in the pooled kernel are ranked
+    // by the CTAs the warp-specialised one would have.
     LmKernelChoice cand[kLmPlainCandidates];
     const int n = lm_candidates(L, cand, kLmPlainCandidates);   // the plain passes
     int best = -1, best_t = 0, best_c = 0, best_w = 0;
@@ -2025,13 +2490,30 @@ size_t lm_smem_bytes(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool rgb
     return per * (size_t)c.slots;
 }
 
+// CTAs of a configuration that fit on an SM; 0: none.  Plain passes: the count the
+// default rule ranks by, CTAs of `threads` threads at 128 registers with `slots`
+// slots of shared memory and control state each (228 KB an SM, 1 KB of it per CTA,
+// 227 KB a CTA at most), of the pooled kernel's configurations too, although it
+// runs one an SM.
 int lm_max_ctas_per_sm(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool rgb)
 {
-    // the Fresnel and horizon variants share the launch configuration
-    KernelFn k = kernel_for(c, false, false, rgb);
-    if(!k || L == 0)
+    if(L == 0)
         return 0;
     const size_t smem = lm_smem_bytes(L, lum_stride, c, rgb);
+    // the Fresnel and horizon variants share the launch configuration
+    KernelFn k = rgb ? nullptr : kernel_for(c, false, false);
+    if(c.pass == kPassPlain || rgb)
+    {
+        if(!k && (!pool_for(c, false, false, rgb) || pool_slots(c.threads / 32 - 1, L, lum_stride, rgb) == 0))
+            return 0;
+        const size_t state = ((rgb ? 2168u : 1400u) * (size_t)c.slots + 16u + 15u) & ~size_t(15);
+        if(smem + state > 227u * 1024u)
+            return 0;
+        return (int)std::min<size_t>(65536u / (128u * (size_t)c.threads),
+                                     228u * 1024u / (((smem + state + 127) & ~size_t(127)) + 1024u));
+    }
+    if(!k)
+        return 0;
     if(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
     {
@@ -2047,19 +2529,42 @@ int lm_max_ctas_per_sm(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool r
     return n;
 }
 
-cudaError_t launch_lm_fit(const LmArgs& args, LmKernelChoice c, int grid, cudaStream_t stream)
+cudaError_t launch_lm_fit(const LmArgs& launch, LmKernelChoice c, int sms, cudaStream_t stream)
 {
-    const bool rgb = args.rgb != 0;
-    KernelFn k = kernel_for(c, args.cfg.fresnel != 1.0f, args.all_up != 0, rgb);
-    if(!k || args.L == 0)
+    LmArgs args = launch;
+    const bool rgb = args.rgb != 0, fresnel = args.cfg.fresnel != 1.0f, all_up = args.all_up != 0;
+    if(args.L == 0 || args.texels == 0 || sms <= 0)
+        return cudaErrorInvalidConfiguration;
+    cudaError_t e;
+    if(const PoolFn k = pool_for(c, fresnel, all_up, rgb))
+    {
+        // a CTA per SM; of its slots as many as there are texels for, and a warp
+        // per share while there are fewer shares than warps
+        const int nw = c.threads / 32 - 1;
+        const uint32_t grid = std::min<uint32_t>((uint32_t)sms, args.texels);
+        const uint32_t fit = pool_slots(nw, args.L, args.lum_stride, rgb);
+        if(fit == 0)
+            return cudaErrorInvalidConfiguration;
+        const uint32_t slots = std::min(fit, (args.texels + grid - 1) / grid);
+        const uint32_t warps = std::min<uint32_t>(kPoolWarps, slots * (uint32_t)nw);
+        const size_t smem = slots * (rgb ? pool_slot_bytes<RgbModel>(nw, args.L, args.lum_stride)
+                                         : pool_slot_bytes<LumModel>(nw, args.L, args.lum_stride));
+        args.counter_base = slots * grid;   // the first texels are dealt out
+        if((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e;
+        k<<<grid, 32 * warps, smem, stream>>>(args, slots);
+        return cudaGetLastError();
+    }
+    KernelFn k = kernel_for(c, fresnel, all_up);
+    const int per_sm = lm_max_ctas_per_sm(args.L, args.lum_stride, c, rgb);
+    if(!k || per_sm <= 0)
         return cudaErrorInvalidConfiguration;
     const size_t smem = lm_smem_bytes(args.L, args.lum_stride, c, rgb);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if(e != cudaSuccess)
+    if((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess ||
+       (e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
         return e;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if(e != cudaSuccess)
-        return e;
+    args.counter_base = 0;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)per_sm * (uint64_t)sms, args.texels);
     k<<<grid, c.threads, smem, stream>>>(args);
     return cudaGetLastError();
 }
