@@ -147,12 +147,12 @@ svf_status mlp_forward(svf_ctx* ctx, const svf_mlp* mlp, const float* X, int row
     {
         const int r = std::min(block, rows - r0);
         const size_t h = (size_t)r0 * kMlpHidden;
-        SVF_CUDA(mlp_gemm(false, true, r, kMlpHidden, kMlpInputs, X + (size_t)r0 * kMlpInputs, kMlpInputs,
+        SVF_CUDA(mlp_gemm(true, r, kMlpHidden, kMlpInputs, X + (size_t)r0 * kMlpInputs, kMlpInputs,
                           w + kMlpW1, kMlpInputs, H1 + h, kMlpHidden, w + kMlpB1, 1, Z1 ? Z1 + h : nullptr, nullptr,
                           ctx->stream));
-        SVF_CUDA(mlp_gemm(false, true, r, kMlpHidden, kMlpHidden, H1 + h, kMlpHidden, w + kMlpW2, kMlpHidden,
+        SVF_CUDA(mlp_gemm(true, r, kMlpHidden, kMlpHidden, H1 + h, kMlpHidden, w + kMlpW2, kMlpHidden,
                           H2 + h, kMlpHidden, w + kMlpB2, 1, Z2 ? Z2 + h : nullptr, nullptr, ctx->stream));
-        SVF_CUDA(mlp_gemm(false, true, r, kMlpOutputs, kMlpHidden, H2 + h, kMlpHidden, w + kMlpW3, kMlpHidden,
+        SVF_CUDA(mlp_gemm(true, r, kMlpOutputs, kMlpHidden, H2 + h, kMlpHidden, w + kMlpW3, kMlpHidden,
                           Y + (size_t)r0 * kMlpOutputs, kMlpOutputs, w + kMlpB3, 0, nullptr, nullptr, ctx->stream));
     }
     return SVF_OK;
@@ -210,7 +210,7 @@ cudaError_t rgb_features(const svf_mlp* mlp, const void* samples, uint32_t sampl
 // Scratch of one training step for `rows` rows (in the context).
 struct MlpScratch
 {
-    DevBuf z1, h1, z2, h2, y, dy, dh2, dh1, dsum, loss;
+    DevBuf z1, h1, z2, h2, y, dy, dh2, dh1, loss;
 };
 
 // One optimiser step on normalised X [rows][96], T [rows][8]: forward, MSE
@@ -228,7 +228,6 @@ svf_status mlp_train_step(svf_ctx* ctx, svf_mlp* mlp, MlpScratch& s, const float
     SVF_TRY(s.dh1.ensure(sizeof(float) * hr));
     SVF_TRY(s.y.ensure(sizeof(float) * rows * kMlpOutputs));
     SVF_TRY(s.dy.ensure(sizeof(float) * rows * kMlpOutputs));
-    SVF_TRY(s.dsum.ensure(sizeof(double) * kMlpHidden));
     SVF_TRY(s.loss.ensure(sizeof(double)));
     float *z1 = s.z1.as<float>(), *h1 = s.h1.as<float>(), *z2 = s.z2.as<float>(), *h2 = s.h2.as<float>();
     float *y = s.y.as<float>(), *dy = s.dy.as<float>(), *dh2 = s.dh2.as<float>(), *dh1 = s.dh1.as<float>();
@@ -237,24 +236,21 @@ svf_status mlp_train_step(svf_ctx* ctx, svf_mlp* mlp, MlpScratch& s, const float
     SVF_TRY(mlp_forward(ctx, mlp, X, rows, z1, h1, z2, h2, y));
     SVF_CUDA(mlp_mse_grad(y, T, rows, kMlpOutputs, dy, s.loss.as<double>(), ctx->stream));
     // layer 3
-    SVF_CUDA(mlp_gemm(true, false, kMlpOutputs, kMlpHidden, rows, dy, kMlpOutputs, h2, kMlpHidden,
-                      g + kMlpW3, kMlpHidden, nullptr, 0, nullptr, nullptr, ctx->stream));
-    SVF_CUDA(mlp_colsum(dy, rows, kMlpOutputs, s.dsum.as<double>(), nullptr, ctx->stream));
-    SVF_CUDA(mlp_to_float(s.dsum.as<double>(), kMlpOutputs, 1.0f, g + kMlpB3, ctx->stream));
-    SVF_CUDA(mlp_gemm(false, false, rows, kMlpHidden, kMlpOutputs, dy, kMlpOutputs, w + kMlpW3, kMlpHidden,
+    SVF_CUDA(mlp_gemm_rows(kMlpOutputs, kMlpHidden, rows, dy, kMlpOutputs, h2, kMlpHidden,
+                      g + kMlpW3, kMlpHidden, ctx->stream));
+    SVF_CUDA(mlp_colsum(dy, rows, kMlpOutputs, nullptr, nullptr, g + kMlpB3, ctx->stream));
+    SVF_CUDA(mlp_gemm(false, rows, kMlpHidden, kMlpOutputs, dy, kMlpOutputs, w + kMlpW3, kMlpHidden,
                       dh2, kMlpHidden, nullptr, 2, nullptr, z2, ctx->stream));
     // layer 2
-    SVF_CUDA(mlp_gemm(true, false, kMlpHidden, kMlpHidden, rows, dh2, kMlpHidden, h1, kMlpHidden,
-                      g + kMlpW2, kMlpHidden, nullptr, 0, nullptr, nullptr, ctx->stream));
-    SVF_CUDA(mlp_colsum(dh2, rows, kMlpHidden, s.dsum.as<double>(), nullptr, ctx->stream));
-    SVF_CUDA(mlp_to_float(s.dsum.as<double>(), kMlpHidden, 1.0f, g + kMlpB2, ctx->stream));
-    SVF_CUDA(mlp_gemm(false, false, rows, kMlpHidden, kMlpHidden, dh2, kMlpHidden, w + kMlpW2, kMlpHidden,
+    SVF_CUDA(mlp_gemm_rows(kMlpHidden, kMlpHidden, rows, dh2, kMlpHidden, h1, kMlpHidden,
+                      g + kMlpW2, kMlpHidden, ctx->stream));
+    SVF_CUDA(mlp_colsum(dh2, rows, kMlpHidden, nullptr, nullptr, g + kMlpB2, ctx->stream));
+    SVF_CUDA(mlp_gemm(false, rows, kMlpHidden, kMlpHidden, dh2, kMlpHidden, w + kMlpW2, kMlpHidden,
                       dh1, kMlpHidden, nullptr, 2, nullptr, z1, ctx->stream));
     // layer 1
-    SVF_CUDA(mlp_gemm(true, false, kMlpHidden, kMlpInputs, rows, dh1, kMlpHidden, X, kMlpInputs, g + kMlpW1,
-                      kMlpInputs, nullptr, 0, nullptr, nullptr, ctx->stream));
-    SVF_CUDA(mlp_colsum(dh1, rows, kMlpHidden, s.dsum.as<double>(), nullptr, ctx->stream));
-    SVF_CUDA(mlp_to_float(s.dsum.as<double>(), kMlpHidden, 1.0f, g + kMlpB1, ctx->stream));
+    SVF_CUDA(mlp_gemm_rows(kMlpHidden, kMlpInputs, rows, dh1, kMlpHidden, X, kMlpInputs, g + kMlpW1,
+                      kMlpInputs, ctx->stream));
+    SVF_CUDA(mlp_colsum(dh1, rows, kMlpHidden, nullptr, nullptr, g + kMlpB1, ctx->stream));
     ++mlp->step;
     SVF_CUDA(mlp_adam(w, g, mlp->m.as<float>(), mlp->v.as<float>(), kMlpParams, lr, mlp->step, sgd, ctx->stream));
     return SVF_OK;
@@ -425,7 +421,7 @@ svf_status svf_mlp_train(svf_ctx* ctx, const float* lp, uint32_t L, const svf_ml
     DevBuf sums;
     SVF_TRY(sums.ensure(sizeof(double) * 2 * kMlpInputs));
     SVF_CUDA(mlp_colsum(X.as<float>(), (int)T, kMlpInputs, sums.as<double>(), sums.as<double>() + kMlpInputs,
-                        ctx->stream));
+                        nullptr, ctx->stream));
     std::vector<double> hs(2 * kMlpInputs);
     std::vector<float> hy((size_t)kMlpOutputs * T);
     SVF_CUDA(cudaMemcpyAsync(hs.data(), sums.p, sizeof(double) * 2 * kMlpInputs, cudaMemcpyDeviceToHost, ctx->stream));

@@ -18,8 +18,9 @@
 //             the eigenvalue nearest 0 is the normal's, the other two give sx,
 //             sy and the tangent frame
 //
-// Training kernels: one tiled FP32 GEMM with transposes and fused bias / GELU /
-// GELU-derivative epilogues, column statistics, the MSE gradient and Adam.
+// Training kernels: tiled FP32 GEMMs with fused bias / GELU / GELU-derivative
+// epilogues, the weight-gradient GEMM over the batch rows, column sums, the MSE
+// gradient and Adam.
 // Inference: the hidden layers on the tcgen05 tensor cores (the BF16x3 GEMM of
 // svf_ndf_tc.cu, FP32 accuracy), the output layer fused into the second
 // layer's epilogue.  The bin features are computed by the luminance pass
@@ -40,8 +41,6 @@ namespace svf
 namespace
 {
 
-constexpr int kTile = 64, kTileK = 16, kGemmThreads = 256;   // 64 x 64 tile, 4 x 4 per thread
-
 __device__ __forceinline__ float gelu(float x)
 {
     const float k = 0.7978845608f;   // sqrt(2 / pi)
@@ -59,62 +58,117 @@ __device__ __forceinline__ float gelu_grad(float x)
 __device__ __forceinline__ float to_f(float x) { return x; }
 __device__ __forceinline__ float to_f(__half x) { return __half2float(x); }
 
-// C[M][N] = op(A) op(B) with op(A)[m][k] = kTA ? A[k][m] : A[m][k] and
-// op(B)[k][n] = kTB ? B[n][k] : B[k][n] (leading dimensions lda, ldb); then
-// + bias[n]; mode 1: Z = C, C = gelu(Z); mode 2: C *= gelu'(Zin).
-template <bool kTA, bool kTB>
-__global__ void __launch_bounds__(kGemmThreads) gemm_kernel(int M, int N, int K, const float* __restrict__ A, int lda,
-                                                            const float* __restrict__ B, int ldb, float* __restrict__ C,
-                                                            int ldc, const float* __restrict__ bias, int mode,
-                                                            float* __restrict__ Z, const float* __restrict__ Zin)
+// C[M][N] = A op(B) with A [M][K] and op(B)[k][n] = kTB ? B[n][k] : B[k][n]
+// (leading dimensions lda, ldb); then + bias[n]; mode 1: Z = C, C = gelu(Z);
+// mode 2: C *= gelu'(Zin).  Every output is one chain of FMAs over k = 0, 1, ..
+// A CTA computes a BM x BN tile, a thread TM x TN of it, in paired FMAs along n (a
+// pair's halves round as the scalar FMA does).  K goes by in tiles of 16, the next
+// one's loads in flight during this one's FMAs.  Bound by the FP32 pipe and the shared
+// loads at 64 x 64 (a step's three forward products over 4096 rows 48 us, 102 with
+// one buffer and scalar loads); smaller tiles where those would leave SMs without
+// one.
+template <bool kTB, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_kernel(int M, int N, int K, const float* __restrict__ A,
+                                                                     int lda, const float* __restrict__ B, int ldb,
+                                                                     float* __restrict__ C, int ldc,
+                                                                     const float* __restrict__ bias, int mode,
+                                                                     float* __restrict__ Z, const float* __restrict__ Zin)
 {
-    __shared__ float As[kTileK][kTile + 1];
-    __shared__ float Bs[kTileK][kTile + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
-    float acc[4][4] = {};
-    for(int k0 = 0; k0 < K; k0 += kTileK)
+    constexpr int BK = 16, T = (BM / TM) * (BN / TN);
+    constexpr int LA = (BM * BK + T - 1) / T, LB = (BN * BK + T - 1) / T;   // elements a thread stages
+    static_assert(TN == 1 || TN % 2 == 0, "paired along n");
+    __shared__ __align__(16) float As[2][BK][BM + 4];
+    __shared__ __align__(16) float Bs[2][BK][BN + 4];
+    const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float ra[LA], rb[LB];
+    auto load = [&](int k0) {
+#pragma unroll
+        for(int q = 0; q < LA; ++q)
+        {
+            const int i = threadIdx.x + q * T, mm = i / BK, kk = i % BK;
+            ra[q] = i < BM * BK && m0 + mm < M && k0 + kk < K ? A[(size_t)(m0 + mm) * lda + k0 + kk] : 0.0f;
+        }
+#pragma unroll
+        for(int q = 0; q < LB; ++q)
+        {
+            const int i = threadIdx.x + q * T;
+            const int nn = kTB ? i / BK : i % BN, kk = kTB ? i % BK : i / BN;
+            rb[q] = i < BN * BK && n0 + nn < N && k0 + kk < K
+                        ? (kTB ? B[(size_t)(n0 + nn) * ldb + k0 + kk] : B[(size_t)(k0 + kk) * ldb + n0 + nn])
+                        : 0.0f;
+        }
+    };
+    auto store = [&](int buf) {
+#pragma unroll
+        for(int q = 0; q < LA; ++q)
+        {
+            const int i = threadIdx.x + q * T;
+            if(i < BM * BK)
+                As[buf][i % BK][i / BK] = ra[q];
+        }
+#pragma unroll
+        for(int q = 0; q < LB; ++q)
+        {
+            const int i = threadIdx.x + q * T;
+            if(i < BN * BK)
+                Bs[buf][kTB ? i % BK : i / BN][kTB ? i / BK : i % BN] = rb[q];
+        }
+    };
+    constexpr int TP = TN == 1 ? 1 : TN / 2;
+    float2 acc[TM][TP];
+#pragma unroll
+    for(int i = 0; i < TM; ++i)
+#pragma unroll
+        for(int j = 0; j < TP; ++j)
+            acc[i][j] = make_float2(0.0f, 0.0f);
+    load(0);
+    store(0);
+    int buf = 0;
+    for(int k0 = 0; k0 < K; k0 += BK, buf ^= 1)
     {
-        for(int i = threadIdx.x; i < kTile * kTileK; i += kGemmThreads)
+        __syncthreads();   // this tile is staged, and the other buffer's last reads are done
+        if(k0 + BK < K)
+            load(k0 + BK);
+#pragma unroll
+        for(int kk = 0; kk < BK; ++kk)
         {
-            const int mm = i / kTileK, kk = i % kTileK;
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? (kTA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]) : 0.0f;
-            const int n = n0 + mm;
-            Bs[kk][mm] = (n < N && k < K) ? (kTB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n]) : 0.0f;
+            float a[TM];
+            float2 b[TP];
+#pragma unroll
+            for(int i = 0; i < TM; ++i)
+                a[i] = As[buf][kk][ty * TM + i];
+            if constexpr(TN == 1)
+                b[0] = make_float2(Bs[buf][kk][tx], 0.0f);
+            else
+#pragma unroll
+                for(int j = 0; j < TP; ++j)
+                    b[j] = *reinterpret_cast<const float2*>(&Bs[buf][kk][tx * TN + 2 * j]);
+#pragma unroll
+            for(int i = 0; i < TM; ++i)
+#pragma unroll
+                for(int j = 0; j < TP; ++j)
+                    if constexpr(TN == 1)
+                        acc[i][j].x = fmaf(a[i], b[j].x, acc[i][j].x);
+                    else
+                        acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
         }
-        __syncthreads();
-#pragma unroll
-        for(int kk = 0; kk < kTileK; ++kk)
-        {
-            float a[4], b[4];
-#pragma unroll
-            for(int i = 0; i < 4; ++i)
-            {
-                a[i] = As[kk][ty * 4 + i];
-                b[i] = Bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for(int i = 0; i < 4; ++i)
-#pragma unroll
-                for(int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
+        if(k0 + BK < K)
+            store(buf ^ 1);
     }
 #pragma unroll
-    for(int i = 0; i < 4; ++i)
+    for(int i = 0; i < TM; ++i)
     {
-        const int m = m0 + ty * 4 + i;
+        const int m = m0 + ty * TM + i;
         if(m >= M)
             continue;
 #pragma unroll
-        for(int j = 0; j < 4; ++j)
+        for(int j = 0; j < TN; ++j)
         {
-            const int n = n0 + tx * 4 + j;
+            const int n = n0 + tx * TN + j;
             if(n >= N)
                 continue;
-            float v = acc[i][j] + (bias ? bias[n] : 0.0f);
+            float v = (j & 1 ? acc[i][j / 2].y : acc[i][j / 2].x) + (bias ? bias[n] : 0.0f);
             if(mode == 1)
             {
                 if(Z)
@@ -128,45 +182,166 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_kernel(int M, int N, int K,
     }
 }
 
-// out[n] = sum_m X[m][n] (and, with out2, sum of squares), in FP64
-__global__ void colsum_kernel(const float* __restrict__ X, int M, int N, double* __restrict__ out,
-                              double* __restrict__ out2)
+constexpr int kRowsStage = 64, kRowsBuffers = 8;
+
+template <int R>
+__device__ __forceinline__ void vec_load(const float* p, float* v)
 {
-    const int n = blockIdx.x;
-    double s = 0.0, s2 = 0.0;
-    for(int m = threadIdx.x; m < M; m += blockDim.x)
+    if constexpr(R == 4)
     {
-        const double v = X[(size_t)m * N + n];
-        s += v;
-        s2 += v * v;
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+        v[2] = x.z;
+        v[3] = x.w;
     }
-    __shared__ double r[2][256];
-    r[0][threadIdx.x] = s;
-    r[1][threadIdx.x] = s2;
-    __syncthreads();
-    for(int o = blockDim.x / 2; o > 0; o >>= 1)
+    else if constexpr(R == 2)
     {
-        if((int)threadIdx.x < o)
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        v[0] = x.x;
+        v[1] = x.y;
+    }
+    else
+        v[0] = *p;
+}
+
+// 16-byte asynchronous copy global -> shared, zero-filled where !ok.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 16u : 0u)
+                 : "memory");
+}
+
+// The weight gradient C[M][N] = A^T B over K batch rows, A [K][M], B [K][N] (row
+// pitches lda, ldb): every output one chain of FMAs over the rows in order, which
+// fixes its rounding and makes the chain the bound (4096 rows x 4 cycles = 8 us).
+// So a CTA takes a small tile (BM x BN, RM x RN outputs a thread) and the launch
+// spreads the outputs over the SMs; 64 rows at a time are staged by 16-byte
+// asynchronous copies, seven stages ahead, each thread's words fixed but for a
+// constant step (with a division per word the staging took most of the issue
+// slots: 95 us).  Widths are multiples of 4.  Over 4096 rows: 256 x 256 525 us in
+// 16 CTAs of 64 x 64, 38 in 128 of 16 x 32; 256 x 96 34 us; 8 x 256 23 us.
+template <int BM, int BN, int RM, int RN>
+__global__ void __launch_bounds__(BM * BN / (RM * RN)) gemm_rows_kernel(int M, int N, int K, const float* __restrict__ A,
+                                                                      int lda, const float* __restrict__ B, int ldb,
+                                                                      float* __restrict__ C, int ldc)
+{
+    constexpr int BK = kRowsStage, kBuffers = kRowsBuffers, T = BM * BN / (RM * RN);
+    constexpr int QA = BM / 4, QB = BN / 4;                 // 16-byte words of a row
+    constexpr int NA = BK * QA / T, NB = BK * QB / T;       // and what a thread copies of a stage
+    static_assert(BK * QA % T == 0 && BK * QB % T == 0 && T % QA == 0 && T % QB == 0, "staging split");
+    extern __shared__ __align__(16) float rows_smem[];
+    const int tx = threadIdx.x % (BN / RN), ty = threadIdx.x / (BN / RN);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float* const as = rows_smem;
+    float* const bs = rows_smem + kBuffers * BK * BM;
+    // this thread's words: column ca / cb of rows ka + j T / QA, kb + j T / QB
+    const int ca = 4 * (threadIdx.x % QA), ka = threadIdx.x / QA, cb = 4 * (threadIdx.x % QB), kb = threadIdx.x / QB;
+    const bool in_m = m0 + ca < M, in_n = n0 + cb < N;
+    const float* src_a = A + (size_t)ka * lda + (in_m ? m0 + ca : 0);
+    const float* src_b = B + (size_t)kb * ldb + (in_n ? n0 + cb : 0);
+    int left = K;   // rows not yet staged
+    auto stage = [&](int buf) {
+        float* da = as + (buf * BK + ka) * BM + ca;
+        float* db = bs + (buf * BK + kb) * BN + cb;
+#pragma unroll
+        for(int j = 0; j < NA; ++j)
         {
-            r[0][threadIdx.x] += r[0][threadIdx.x + o];
-            r[1][threadIdx.x] += r[1][threadIdx.x + o];
+            const bool ok = in_m && ka + j * (T / QA) < left;
+            cp_async16(da + j * (T / QA) * BM, ok ? src_a + (size_t)(j * (T / QA)) * lda : A, ok);
+        }
+#pragma unroll
+        for(int j = 0; j < NB; ++j)
+        {
+            const bool ok = in_n && kb + j * (T / QB) < left;
+            cp_async16(db + j * (T / QB) * BN, ok ? src_b + (size_t)(j * (T / QB)) * ldb : B, ok);
+        }
+        src_a += (size_t)BK * lda;
+        src_b += (size_t)BK * ldb;
+        left -= BK;
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    float acc[RM][RN] = {};
+#pragma unroll
+    for(int b = 0; b < kBuffers - 1; ++b)
+        stage(b);
+    int buf = 0;
+    for(int k0 = 0; k0 < K; k0 += BK)
+    {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBuffers - 2) : "memory");
+        __syncthreads();   // this buffer has arrived, and the one staged next is read
+        stage(buf == 0 ? kBuffers - 1 : buf - 1);
+        const float* ta = as + buf * BK * BM + ty * RM;
+        const float* tb = bs + buf * BK * BN + tx * RN;
+#pragma unroll
+        for(int kk = 0; kk < BK; ++kk)
+        {
+            float a[RM], b[RN];
+            vec_load<RM>(ta + kk * BM, a);
+            vec_load<RN>(tb + kk * BN, b);
+#pragma unroll
+            for(int i = 0; i < RM; ++i)
+#pragma unroll
+                for(int j = 0; j < RN; ++j)
+                    acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        buf = buf == kBuffers - 1 ? 0 : buf + 1;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");   // (no copy outlives the CTA)
+#pragma unroll
+    for(int i = 0; i < RM; ++i)
+#pragma unroll
+        for(int j = 0; j < RN; ++j)
+        {
+            const int m = m0 + ty * RM + i, n = n0 + tx * RN + j;
+            if(m < M && n < N)
+                C[(size_t)m * ldc + n] = acc[i][j];
+        }
+}
+
+// out[n] = sum_m X[m][n] (and, with out2, sum of squares), in FP64: 256 sums per
+// column, of the rows m = t (mod 256) in order, folded by halves.  A CTA takes 8
+// columns (whole 32-byte sectors of every row), a thread one column's sums t =
+// tid / 8 and t + 128; out_f takes the sums as floats.
+__global__ void __launch_bounds__(1024) colsum_kernel(const float* __restrict__ X, int M, int N, double* __restrict__ out,
+                                                      double* __restrict__ out2, float* __restrict__ out_f)
+{
+    __shared__ double r[2][256][8];
+    const int c = threadIdx.x & 7, t0 = threadIdx.x >> 3, n = blockIdx.x * 8 + c;
+    for(int t = t0; t < 256; t += 128)
+    {
+        double s = 0.0, s2 = 0.0;
+        if(n < N)
+#pragma unroll 4
+            for(int m = t; m < M; m += 256)
+            {
+                const double v = X[(size_t)m * N + n];
+                s += v;
+                s2 += v * v;
+            }
+        r[0][t][c] = s;
+        r[1][t][c] = s2;
+    }
+    __syncthreads();
+    for(int o = 128; o > 0; o >>= 1)
+    {
+        if(t0 < o)
+        {
+            r[0][t0][c] += r[0][t0 + o][c];
+            r[1][t0][c] += r[1][t0 + o][c];
         }
         __syncthreads();
     }
-    if(threadIdx.x == 0)
+    if(t0 == 0 && n < N)
     {
-        out[n] = r[0][0];
+        if(out)
+            out[n] = r[0][0][c];
         if(out2)
-            out2[n] = r[1][0];
+            out2[n] = r[1][0][c];
+        if(out_f)
+            out_f[n] = (float)r[0][0][c];
     }
-}
-
-// FP32 copy of a double vector
-__global__ void to_float_kernel(const double* __restrict__ x, int n, float scale, float* __restrict__ y)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i < n)
-        y[i] = (float)(x[i] * scale);
 }
 
 // X[m][n] = (X[m][n] - mean[n]) * rstd[n]
@@ -467,35 +642,73 @@ inline unsigned blocks_for(size_t n, unsigned threads) { return (unsigned)((n + 
 
 } // namespace
 
-cudaError_t mlp_gemm(bool ta, bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-                     float* C, int ldc, const float* bias, int mode, float* Z, const float* Zin, cudaStream_t stream)
+namespace
 {
-    dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
+
+template <bool kTB, int BM, int BN, int TM, int TN>
+cudaError_t launch_gemm(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                        const float* bias, int mode, float* Z, const float* Zin, cudaStream_t stream)
+{
+    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if(grid.y > 65535)
         return cudaErrorInvalidValue;
-#define SVF_GEMM(TA, TB) \
-    gemm_kernel<TA, TB><<<grid, kGemmThreads, 0, stream>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin)
-    if(!ta && tb)
-        SVF_GEMM(false, true);
-    else if(ta && !tb)
-        SVF_GEMM(true, false);
-    else if(!ta && !tb)
-        SVF_GEMM(false, false);
-    else
-        return cudaErrorInvalidValue;
-#undef SVF_GEMM
+    gemm_kernel<kTB, BM, BN, TM, TN>
+        <<<grid, (BM / TM) * (BN / TN), 0, stream>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin);
     return cudaGetLastError();
 }
 
-cudaError_t mlp_colsum(const float* X, int M, int N, double* sum, double* sumsq, cudaStream_t stream)
+// Tiles: a column of 8 outputs (the network's last layer) takes 8-wide tiles; else
+// 64 x 64 while they make a CTA for every SM, 32 x 32 below.
+template <bool kTB, class... Args>
+cudaError_t pick_gemm(int M, int N, Args... args)
 {
-    colsum_kernel<<<N, 256, 0, stream>>>(X, M, N, sum, sumsq);
+    if(N <= 8)
+        return launch_gemm<kTB, 32, 8, 1, 1>(M, N, args...);
+    if((int64_t)((M + 63) / 64) * ((N + 63) / 64) >= 148)
+        return launch_gemm<kTB, 64, 64, 4, 4>(M, N, args...);
+    return launch_gemm<kTB, 32, 32, 2, 4>(M, N, args...);
+}
+
+template <int BM, int BN, int RM, int RN>
+cudaError_t launch_rows(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                        cudaStream_t stream)
+{
+    const size_t smem = sizeof(float) * kRowsBuffers * kRowsStage * (BM + BN);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<BM, BN, RM, RN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if(e != cudaSuccess)
+        return e;
+    gemm_rows_kernel<BM, BN, RM, RN><<<dim3((N + BN - 1) / BN, (M + BM - 1) / BM), BM * BN / (RM * RN), smem, stream>>>(
+        M, N, K, A, lda, B, ldb, C, ldc);
     return cudaGetLastError();
 }
 
-cudaError_t mlp_to_float(const double* x, int n, float scale, float* y, cudaStream_t stream)
+} // namespace
+
+cudaError_t mlp_gemm(bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                     const float* bias, int mode, float* Z, const float* Zin, cudaStream_t stream)
 {
-    to_float_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(x, n, scale, y);
+    return tb ? pick_gemm<true>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream)
+              : pick_gemm<false>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream);
+}
+
+cudaError_t mlp_gemm_rows(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
+                          cudaStream_t stream)
+{
+    if(M % 4 || N % 4 || lda % 4 || ldb % 4 || (reinterpret_cast<uintptr_t>(A) & 15u) ||
+       (reinterpret_cast<uintptr_t>(B) & 15u))
+        return cudaErrorInvalidValue;   // (the 16-byte copies; every layer's widths are multiples of 8)
+    // the largest tile that makes a CTA for at least half the SMs
+    if((int64_t)M * N >= 148 * 16 * 32 / 2)
+        return launch_rows<16, 32, 2, 2>(M, N, K, A, lda, B, ldb, C, ldc, stream);
+    if((int64_t)M * N >= 148 * 16 * 16 / 2)
+        return launch_rows<16, 16, 2, 2>(M, N, K, A, lda, B, ldb, C, ldc, stream);
+    return launch_rows<8, 8, 1, 1>(M, N, K, A, lda, B, ldb, C, ldc, stream);
+}
+
+cudaError_t mlp_colsum(const float* X, int M, int N, double* sum, double* sumsq, float* sum_f, cudaStream_t stream)
+{
+    colsum_kernel<<<(N + 7) / 8, 1024, 0, stream>>>(X, M, N, sum, sumsq, sum_f);
     return cudaGetLastError();
 }
 
