@@ -15,17 +15,21 @@
 // the exponentials are CUDA's expf (within 2 ulp of libm's), so those samples
 // agree to a few ulp.
 //
-// Work split: a CTA of 128 threads owns 128 consecutive pairs lv (one per
-// thread) and TX texels (16 for half planes, whose accumulators then leave room
-// for more resident CTAs; 32 for float planes).  Per chunk of 32 components the CTA stages, with
-// coalesced loads, the 128 U rows (transposed, padded: a thread reads its pair's
-// value conflict-free) and the TX texels' SxV rows (transposed: a thread reads
-// TX of them with vector broadcasts) in shared memory.  Half planes accumulate
-// with FMAs (a product of two halves is exact in float, so the FMA rounds as the
-// reference's separate multiply and add do); float and double planes need the
-// separate multiply and add.  Writes: a warp stores 32 consecutive pairs x 3
-// channels of one texel at a time (384 contiguous bytes in FP32).  Bound by
-// the FP32 pipe for K >= ~20 components, by the HBM write otherwise.
+// Half and float planes (btf_decode_tile_kernel): a CTA of 256 threads decodes 128
+// pairs x 64 texels, a thread 8 x 4 of them in all three channels: 96 sums, so that
+// its samples leave with their channels together and two CTAs share an SM (one
+// stores while the other multiplies).  What bounds it is the 32 words a clock that
+// shared memory returns to registers, whether or not lanes ask for the same word: 12
+// words for 32 products, 82 % of that rate against 55 % of the FP32 pipe's.  8 x 8 a
+// thread (16 words for 64 products) needs 192 sums and leaves one CTA: 9.25 ms where
+// this takes 8.45.  Half planes accumulate with FMAs (a product of two halves is exact
+// in float, so the FMA rounds as the reference's separate multiply and add do), two
+// pairs to an instruction; float planes multiply, then add; each sum keeps its order.
+// Measured, 81 directions, half planes of 48 components: 400 x 400 texels 8.6 ms
+// (17.2 with a thread to one pair x 16 texels and 128 threads), 64 x 64 0.25 (0.48),
+// one texel 35 us (38); float planes, 400 x 400: 13.9 ms (24.7).
+// Double planes (btf_decode_kernel): a thread takes one pair, a CTA 128 pairs and
+// 16 texels.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -45,25 +49,42 @@ __device__ __forceinline__ float elem(const float* p, uint64_t i) { return p[i];
 __device__ __forceinline__ double elem(const double* p, uint64_t i) { return p[i]; }
 
 // sum + u * v with the product rounded first (no contraction into an FMA,
-// which would round once); for half elements the product is exact in float and
-// an FMA gives the same result.
-template <typename T>
-__device__ __forceinline__ float madd(float sum, float u, float v) { return __fadd_rn(sum, __fmul_rn(u, v)); }
-template <>
-__device__ __forceinline__ float madd<__half>(float sum, float u, float v) { return __fmaf_rn(u, v, sum); }
-template <typename T>
+// which would round once).
 __device__ __forceinline__ double madd(double sum, double u, double v) { return __dadd_rn(sum, __dmul_rn(u, v)); }
 
-// The epilogue of a CTA: colour model 11 and DRR, then the TX texels' samples
-// of its 128 pairs, a warp storing 32 consecutive pairs x RGB of one texel at
-// a time.
+// Colour model 11 (log-YUV) and DRR on a sample's three decoded values.
+__device__ __forceinline__ void to_sample(const BtfDecodeArgs& a, float* v)
+{
+    const float eps = 1e-5f;
+    if(a.color_model == 11)
+    {
+        // btf.hh:522-531 and YUVToRGB (spectrum.hh:344-350): dot products
+        // with the conversion's columns, left to right, then a clamp to [0, 1]
+        const float Y = __fsub_rn(expf(v[0]), eps);
+        const float U = __fadd_rn(__fmul_rn(v[1], Y), eps);
+        const float V = __fadd_rn(__fmul_rn(v[2], Y), eps);
+        v[0] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, 0.0f)), __fmul_rn(V, 1.13983f));
+        v[1] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, -0.39465f)), __fmul_rn(V, -0.5806f));
+        v[2] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, 2.03211f)), __fmul_rn(V, 0.0f));
+        // Clamp (functions.hh:156-159)
+#pragma unroll
+        for(int i = 0; i < 3; ++i)
+            v[i] = v[i] <= 0.0f ? 0.0f : (v[i] >= 1.0f ? 1.0f : v[i]);
+    }
+    if(a.drr)
+#pragma unroll
+        for(int i = 0; i < 3; ++i)
+            v[i] = __fsub_rn(expf(v[i]), eps);
+}
+
+// The epilogue of a CTA of btf_decode_kernel: the TX texels' samples of its 128
+// pairs, a warp storing 32 consecutive pairs x RGB of one texel at a time.
 template <typename Acc, int TX>
 __device__ __forceinline__ void store_texels(const BtfDecodeArgs& a, const Acc (&acc)[3][TX], uint64_t t0,
                                              uint32_t lv0)
 {
     __shared__ float s_out[kThreads / 32][96];   // one texel's 32 pairs x RGB per warp
     const uint64_t t_end = a.first + a.count;
-    const float eps = 1e-5f;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t lv_w = lv0 + warp * 32;   // the warp's first pair
     const uint32_t nvalid = lv_w >= a.N ? 0u : (a.N - lv_w < 32u ? a.N - lv_w : 32u);
@@ -73,37 +94,13 @@ __device__ __forceinline__ void store_texels(const BtfDecodeArgs& a, const Acc (
         const uint64_t t = t0 + j;
         if(t >= t_end)
             break;   // (the same for the whole CTA)
-        float r = (float)acc[0][j], g = (float)acc[1][j], b = (float)acc[2][j];
-        if(a.color_model == 11)
-        {
-            // btf.hh:522-531 and YUVToRGB (spectrum.hh:344-350): dot products
-            // with the conversion's columns, left to right, then a clamp to [0, 1]
-            const float Y = __fsub_rn(expf(r), eps);
-            const float U = __fadd_rn(__fmul_rn(g, Y), eps);
-            const float V = __fadd_rn(__fmul_rn(b, Y), eps);
-            float o[3];
-            o[0] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, 0.0f)), __fmul_rn(V, 1.13983f));
-            o[1] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, -0.39465f)), __fmul_rn(V, -0.5806f));
-            o[2] = __fadd_rn(__fadd_rn(__fmul_rn(Y, 1.0f), __fmul_rn(U, 2.03211f)), __fmul_rn(V, 0.0f));
-            // Clamp (functions.hh:156-159)
-#pragma unroll
-            for(int i = 0; i < 3; ++i)
-                o[i] = o[i] <= 0.0f ? 0.0f : (o[i] >= 1.0f ? 1.0f : o[i]);
-            r = o[0];
-            g = o[1];
-            b = o[2];
-        }
-        if(a.drr)
-        {
-            r = __fsub_rn(expf(r), eps);
-            g = __fsub_rn(expf(g), eps);
-            b = __fsub_rn(expf(b), eps);
-        }
+        float v[3] = { (float)acc[0][j], (float)acc[1][j], (float)acc[2][j] };
+        to_sample(a, v);
         // the warp's 32 samples are 96 consecutive values: stage them and store
         // them lane-consecutive (each store instruction covers 32 neighbours)
-        s_out[warp][3 * lane] = r;
-        s_out[warp][3 * lane + 1] = g;
-        s_out[warp][3 * lane + 2] = b;
+        s_out[warp][3 * lane] = v[0];
+        s_out[warp][3 * lane + 1] = v[1];
+        s_out[warp][3 * lane + 2] = v[2];
         __syncwarp();
         const uint64_t o = ((t - a.first) * a.N + lv_w) * 3;
         if(a.out_type == SVF_SAMPLES_F16)
@@ -177,150 +174,233 @@ __global__ void __launch_bounds__(kThreads) btf_decode_kernel(BtfDecodeArgs a, u
                 const Acc u = s_u[kk][threadIdx.x];
 #pragma unroll
                 for(int j = 0; j < TX; ++j)
-                    acc[c][j] = madd<T>(acc[c][j], u, s_sxv[kk][j]);
+                    acc[c][j] = madd(acc[c][j], u, s_sxv[kk][j]);
             }
         }
     }
     store_texels<Acc, TX>(a, acc, t0, lv0);
 }
 
-// 4-byte asynchronous copy global -> shared (cp.async, L1-allocating), the
-// bytes past src_bytes (0, 2 or 4) zero-filled.
-__device__ __forceinline__ void cp_async4(void* dst, const void* src, uint32_t src_bytes)
-{
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+constexpr int kTilePairs = 128, kTileTexels = 64, kTileThreads = 256, kTileK = 16;
 
-// Half planes with 4-byte aligned rows: the same sums as btf_decode_kernel, the
-// staging double-buffered so that the next chunk's loads run under this
-// chunk's FMAs.  U arrives by cp.async as half2 words (components k, k+1 of a
-// pair's row; word rows padded to 130 so that the copies of a warp, two pairs x
-// 16 words, hit 32 banks, and a thread's read of its pair is conflict-free);
-// SxV through registers, converted to float and transposed as before.  The
-// chunk sequence runs over the three channels, each channel's accumulator row
-// selected by a compile-time switch.
-template <int TX>
-__global__ void __launch_bounds__(kThreads) btf_decode_half_async_kernel(BtfDecodeArgs a, uint64_t t_begin)
+__device__ __forceinline__ float2 pair_madd(float2 sum, float2 u, float v, const __half*)
 {
-    constexpr int kWords = kChunk / 2, kRowWords = kThreads + 2;
-    constexpr int kSx = TX * kChunk / kThreads;   // SxV elements a thread stages per chunk
-    static_assert(TX * kChunk % kThreads == 0, "SxV staging split");
-    __shared__ uint32_t s_u[2][kWords][kRowWords];
-    __shared__ __align__(16) float s_sxv[2][kChunk][TX + 4];
-    __shared__ uint64_t s_col[TX];
-    const uint32_t lv0 = blockIdx.x * kThreads;
-    const uint64_t t0 = t_begin + (uint64_t)blockIdx.y * TX;
-    const uint64_t t_end = a.first + a.count;
-    if(threadIdx.x < TX)
+    return __ffma2_rn(u, make_float2(v, v), sum);
+}
+// (the paired multiply and add would be contracted)
+__device__ __forceinline__ float2 pair_madd(float2 sum, float2 u, float v, const float*)
+{
+    return make_float2(__fadd_rn(sum.x, __fmul_rn(u.x, v)), __fadd_rn(sum.y, __fmul_rn(u.y, v)));
+}
+
+// kE consecutive elements of a row, as they lie in the file.
+template <typename T, int kE>
+struct alignas(sizeof(T) * kE < 16 ? sizeof(T) * kE : 16) Elems { T v[kE]; };
+
+// Elements k0 .. k0 + kE - 1 of a row of K, 0 past K.  kWide: the row is aligned to
+// Elems<T, kE> at k0 and K is a multiple of kE.
+template <bool kWide, typename T, int kE>
+__device__ __forceinline__ void load_elems(const T* row, uint32_t k0, uint32_t K, bool ok, Elems<T, kE>& e)
+{
+    if constexpr(kWide)
     {
-        const uint64_t t = t0 + threadIdx.x;
-        const uint64_t y = t / a.width, x = t - y * a.width;
-        s_col[threadIdx.x] = t < t_end ? (a.height - 1 - y) * a.width + x : ~0ull;
+        if(ok && k0 < K)
+            e = *reinterpret_cast<const Elems<T, kE>*>(row + k0);
+        else
+#pragma unroll
+            for(int i = 0; i < kE; ++i)
+                e.v[i] = T(0.0f);
     }
-    __syncthreads();
-    // chunks: (channel, first component)
-    uint32_t nq[3];
+    else
+#pragma unroll
+        for(int i = 0; i < kE; ++i)
+            e.v[i] = ok && k0 + i < K ? row[k0 + i] : T(0.0f);
+}
+
+// Column swaps of the staged operands' upper 8 rows, so that the lanes that stage
+// consecutive pieces of one row do not meet in a bank.
+__device__ __forceinline__ int swap_u(int kk) { return kk >= 8 ? 16 : 0; }
+__device__ __forceinline__ int swap_s(int kk) { return kk >= 8 ? 8 : 0; }
+
+// Thread (tl, tx): pairs tl * 4 + {0..3} and 64 + tl * 4 + {0..3}, texels tx * 4 +
+// {0..3}; a warp is 8 tl x 4 tx.  The components go by in tiles of 16 through two
+// shared buffers, the next tile's elements in registers during this one's products.
+template <typename T, bool kWide>
+__global__ void __launch_bounds__(kTileThreads, 2) btf_decode_tile_kernel(BtfDecodeArgs a, uint64_t t_begin)
+{
+    constexpr int TX = 4, kTexels = kTileTexels;
+    constexpr int kS = kTexels * kTileK / kTileThreads;   // elements of SxV a thread stages of a tile
+    struct Operands
+    {
+        float u[2][kTileK][kTilePairs + 4];
+        float s[2][kTileK][kTexels + 4];
+    };
+    union Shared   // the samples leave through the operands' memory
+    {
+        Operands op;
+        float out[kTileThreads / 32][4][2][96];
+    };
+    __shared__ __align__(16) unsigned char s_mem[sizeof(Shared)];
+    Shared& sh = *reinterpret_cast<Shared*>(s_mem);
+    const uint32_t lv0 = blockIdx.x * kTilePairs;
+    const uint64_t t0 = t_begin + (uint64_t)blockIdx.y * kTexels;
+    const uint64_t t_end = a.first + a.count;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tl = (lane & 7) + 8 * (warp & 1), tx = (lane >> 3) + 4 * (warp >> 1);
+    // staging: U elements 8 pu .. of pair lu; SxV elements kS ps .. of texel ls, whose
+    // file column is row H - 1 - y
+    const int lu = threadIdx.x / 2, pu = threadIdx.x % 2;
+    const int ls = threadIdx.x / (kTileK / kS), ps = threadIdx.x % (kTileK / kS);
+    const bool u_ok = lv0 + lu < a.N, s_ok = t0 + ls < t_end;
+    uint64_t col = 0;
+    if(s_ok)
+    {
+        const uint64_t t = t0 + ls, y = t / a.width;
+        col = (a.height - 1 - y) * a.width + (t - y * a.width);
+    }
+    float2 acc[3][4][TX];
+#pragma unroll
     for(int c = 0; c < 3; ++c)
-        nq[c] = (a.k[c] + kChunk - 1) / kChunk;
-    const uint32_t n_chunks = nq[0] + nq[1] + nq[2];
-    auto chunk = [&](uint32_t q, int& c, uint32_t& k0) {
-        c = q < nq[0] ? 0 : (q < nq[0] + nq[1] ? 1 : 2);
-        k0 = (q - (c == 0 ? 0 : (c == 1 ? nq[0] : nq[0] + nq[1]))) * kChunk;
-    };
-    // U: thread t copies words w = t % 16 of rows t / 16 + 8 i
-    const int uw = threadIdx.x % kWords, ur = threadIdx.x / kWords;
-    auto issue_u = [&](uint32_t q, int buf) {
-        int c;
-        uint32_t k0;
-        chunk(q, c, k0);
-        const __half* U = static_cast<const __half*>(a.u[c]);
-        const uint32_t K = a.k[c];
-        const uint32_t k = k0 + 2 * uw;
-        const uint32_t bytes = k + 1 < K ? 4u : (k < K ? 2u : 0u);
-        for(int row = ur; row < kThreads; row += kThreads / kWords)
-        {
-            const bool ok = lv0 + row < a.N && bytes > 0;
-            const __half* src = ok ? U + (uint64_t)(lv0 + row) * a.u_row[c] + k : U;
-            cp_async4(&s_u[buf][uw][row], src, ok ? bytes : 0u);
-        }
-    };
-    // SxV: thread t loads component t % 32 of texels t / 32 + 4 i
-    const int sk = threadIdx.x % kChunk, sj = threadIdx.x / kChunk;
-    float sx[kSx];
-    auto load_sx = [&](uint32_t q) {
-        int c;
-        uint32_t k0;
-        chunk(q, c, k0);
-        const __half* S = static_cast<const __half*>(a.sxv[c]);
-        const bool k_ok = k0 + sk < a.k[c];
 #pragma unroll
-        for(int i = 0; i < kSx; ++i)
-        {
-            const uint64_t col = s_col[sj + i * (kThreads / kChunk)];
-            sx[i] = (col != ~0ull && k_ok) ? __half2float(S[col * a.sxv_row[c] + k0 + sk]) : 0.0f;
-        }
-    };
-    auto store_sx = [&](int buf) {
-#pragma unroll
-        for(int i = 0; i < kSx; ++i)
-            s_sxv[buf][sk][sj + i * (kThreads / kChunk)] = sx[i];
-    };
-    float acc[3][TX];
-#pragma unroll
-    for(int c = 0; c < 3; ++c)
-#pragma unroll
-        for(int j = 0; j < TX; ++j)
-            acc[c][j] = 0.0f;
-    auto compute = [&](float (&ac)[TX], int buf, uint32_t n) {
-        for(uint32_t kk = 0; kk < n; kk += 2)
-        {
-            const uint32_t w = s_u[buf][kk >> 1][threadIdx.x];
-            const float u0 = __half2float(__ushort_as_half((unsigned short)(w & 0xffffu)));
-            const float u1 = __half2float(__ushort_as_half((unsigned short)(w >> 16)));
+        for(int i = 0; i < 4; ++i)
 #pragma unroll
             for(int j = 0; j < TX; ++j)
-                ac[j] = __fmaf_rn(u0, s_sxv[buf][kk][j], ac[j]);
-            if(kk + 1 < n)
+                acc[c][i][j] = make_float2(0.0f, 0.0f);
+    int buf = 0;
+#pragma unroll
+    for(int c = 0; c < 3; ++c)
+    {
+        const T* U = static_cast<const T*>(a.u[c]) + (uint64_t)(u_ok ? lv0 + lu : 0) * a.u_row[c] + 8 * pu;
+        const T* S = static_cast<const T*>(a.sxv[c]) + col * a.sxv_row[c] + kS * ps;
+        const uint32_t K = a.k[c], Ku = K > 8u * pu ? K - 8 * pu : 0, Ks = K > (uint32_t)(kS * ps) ? K - kS * ps : 0;
+        Elems<T, 8> ru;
+        Elems<T, kS> rs;
+        load_elems<kWide>(U, 0, Ku, u_ok, ru);
+        load_elems<kWide>(S, 0, Ks, s_ok, rs);
+        for(uint32_t k0 = 0; k0 < K; k0 += kTileK)
+        {
+#pragma unroll
+            for(int i = 0; i < 8; ++i)
+                sh.op.u[buf][8 * pu + i][lu ^ swap_u(8 * pu)] = elem(ru.v, i);
+#pragma unroll
+            for(int i = 0; i < kS; ++i)
+                sh.op.s[buf][kS * ps + i][ls ^ swap_s(kS * ps)] = elem(rs.v, i);
+            __syncthreads();   // (a buffer is written again two tiles on, past the next barrier)
+            if(k0 + kTileK < K)
+            {
+                load_elems<kWide>(U, k0 + kTileK, Ku, u_ok, ru);
+                load_elems<kWide>(S, k0 + kTileK, Ks, s_ok, rs);
+            }
+            const uint32_t n = K - k0 < (uint32_t)kTileK ? K - k0 : (uint32_t)kTileK;
+            auto step = [&](uint32_t kk) {
+                const float4 u0 = *reinterpret_cast<const float4*>(&sh.op.u[buf][kk][(4 * tl) ^ swap_u(kk)]);
+                const float4 u1 = *reinterpret_cast<const float4*>(&sh.op.u[buf][kk][64 + ((4 * tl) ^ swap_u(kk))]);
+                const float2 u[4] = { make_float2(u0.x, u0.y), make_float2(u0.z, u0.w), make_float2(u1.x, u1.y),
+                                      make_float2(u1.z, u1.w) };
+                const float4 s0 = *reinterpret_cast<const float4*>(&sh.op.s[buf][kk][(4 * tx) ^ swap_s(kk)]);
+                const float v[TX] = { s0.x, s0.y, s0.z, s0.w };
 #pragma unroll
                 for(int j = 0; j < TX; ++j)
-                    ac[j] = __fmaf_rn(u1, s_sxv[buf][kk + 1][j], ac[j]);
+#pragma unroll
+                    for(int i = 0; i < 4; ++i)
+                        acc[c][i][j] = pair_madd(acc[c][i][j], u[i], v[j], static_cast<const T*>(nullptr));
+            };
+            if(n == (uint32_t)kTileK)
+            {
+#pragma unroll 8
+                for(uint32_t kk = 0; kk < (uint32_t)kTileK; ++kk)
+                    step(kk);
+            }
+            else
+                for(uint32_t kk = 0; kk < n; ++kk)
+                    step(kk);
+            buf ^= 1;
         }
-    };
-    issue_u(0, 0);
-    cp_async_commit();
-    load_sx(0);
-    for(uint32_t q = 0; q < n_chunks; ++q)
-    {
-        const int buf = q & 1;
-        store_sx(buf);
-        if(q + 1 < n_chunks)
-        {
-            issue_u(q + 1, buf ^ 1);
-            cp_async_commit();
-            load_sx(q + 1);
-            cp_async_wait<1>();
-        }
-        else
-            cp_async_wait<0>();
-        __syncthreads();
-        int c;
-        uint32_t k0;
-        chunk(q, c, k0);
-        const uint32_t n = a.k[c] - k0 < (uint32_t)kChunk ? a.k[c] - k0 : (uint32_t)kChunk;
-        if(c == 0)
-            compute(acc[0], buf, n);
-        else if(c == 1)
-            compute(acc[1], buf, n);
-        else
-            compute(acc[2], buf, n);
-        __syncthreads();
     }
-    cp_async_wait<0>();   // (no copy outlives the CTA, also when there was no chunk)
-    store_texels<float, TX>(a, acc, t0, lv0);
+    // samples out: two of a warp's texels at a time through shared memory, so that its
+    // stores are consecutive
+    __syncthreads();
+    float(*out)[2][96] = sh.out[warp];
+#pragma unroll
+    for(int j = 0; j < TX; ++j)
+    {
+#pragma unroll
+        for(int g = 0; g < 2; ++g)
+        {
+            float v[12];   // the group's four pairs
+#pragma unroll
+            for(int i = 0; i < 2; ++i)
+#pragma unroll
+                for(int c = 0; c < 3; ++c)
+                {
+                    v[6 * i + c] = acc[c][2 * g + i][j].x;
+                    v[6 * i + 3 + c] = acc[c][2 * g + i][j].y;
+                }
+#pragma unroll
+            for(int p = 0; p < 4; ++p)
+                to_sample(a, v + 3 * p);
+#pragma unroll
+            for(int w = 0; w < 3; ++w)
+                *reinterpret_cast<float4*>(&out[lane >> 3][g][12 * (lane & 7) + 4 * w]) =
+                    make_float4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for(int r = 0; r < 4; ++r)
+        {
+            const uint64_t t = t0 + (uint64_t)(4 * (warp >> 1) + r) * TX + j;
+            if(t >= t_end)
+                continue;
+#pragma unroll
+            for(int g = 0; g < 2; ++g)
+            {
+                const uint32_t lv = lv0 + 64 * g + 32 * (warp & 1);
+                const uint32_t values = lv >= a.N ? 0 : a.N - lv < 32 ? 3 * (a.N - lv) : 96;
+                const uint64_t o = ((t - a.first) * a.N + lv) * 3;
+                if(a.out_type == SVF_SAMPLES_F16)
+                {
+#pragma unroll
+                    for(uint32_t e = lane; e < 96; e += 32)
+                        if(e < values)
+                            static_cast<__half*>(a.out)[o + e] = __float2half_rn(out[r][g][e]);
+                }
+                else
+#pragma unroll
+                    for(uint32_t e = lane; e < 96; e += 32)
+                        if(e < values)
+                            static_cast<float*>(a.out)[o + e] = out[r][g][e];
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <typename T, bool kWide>
+cudaError_t launch_tiles_of(const BtfDecodeArgs& a, cudaStream_t stream)
+{
+    constexpr uint64_t texels = kTileTexels, per_launch = 65535ull * texels;   // grid.y limit
+    for(uint64_t t = a.first; t < a.first + a.count; t += per_launch)
+    {
+        const uint64_t n = a.first + a.count - t < per_launch ? a.first + a.count - t : per_launch;
+        const dim3 grid((a.N + kTilePairs - 1) / kTilePairs, (unsigned)((n + texels - 1) / texels));
+        btf_decode_tile_kernel<T, kWide><<<grid, kTileThreads, 0, stream>>>(a, t);
+        const cudaError_t e = cudaGetLastError();
+        if(e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
+template <typename T>
+cudaError_t launch_tiles(const BtfDecodeArgs& a, cudaStream_t stream)
+{
+    // Elems loads of 8 components want aligned rows of whole groups; 47 components, an
+    // element at a time, take 10.1 ms where 48 take 8.6
+    bool wide = true;
+    for(int c = 0; c < 3; ++c)
+        wide = wide && a.k[c] % 8 == 0 && a.u_row[c] * sizeof(T) % 16 == 0 && a.sxv_row[c] * sizeof(T) % 16 == 0 &&
+               (uintptr_t)a.u[c] % 16 == 0 && (uintptr_t)a.sxv[c] % 16 == 0;
+    return wide ? launch_tiles_of<T, true>(a, stream) : launch_tiles_of<T, false>(a, stream);
 }
 
 template <typename T, typename Acc, int TX>
@@ -347,28 +427,8 @@ cudaError_t launch_btf_decode(const BtfDecodeArgs& a, cudaStream_t stream)
         return cudaSuccess;
     switch(a.data_size)
     {
-    case 2:
-    {
-        // the asynchronous staging wants every U row 4-byte aligned
-        bool aligned = true;
-        for(int c = 0; c < 3; ++c)
-            aligned = aligned && (a.u_row[c] % 2 == 0) && ((uintptr_t)a.u[c] % 4 == 0);
-        if(!aligned)
-            return launch_typed<__half, float, 16>(a, stream);
-        constexpr int TX = 16;
-        const uint64_t per_launch = 65535ull * TX;
-        for(uint64_t t = a.first; t < a.first + a.count; t += per_launch)
-        {
-            const uint64_t n = a.first + a.count - t < per_launch ? a.first + a.count - t : per_launch;
-            dim3 grid((a.N + kThreads - 1) / kThreads, (unsigned)((n + TX - 1) / TX));
-            btf_decode_half_async_kernel<TX><<<grid, kThreads, 0, stream>>>(a, t);
-            const cudaError_t e = cudaGetLastError();
-            if(e != cudaSuccess)
-                return e;
-        }
-        return cudaSuccess;
-    }
-    case 4: return launch_typed<float, float, 32>(a, stream);
+    case 2: return launch_tiles<__half>(a, stream);
+    case 4: return launch_tiles<float>(a, stream);
     case 8: return launch_typed<double, double, 16>(a, stream);
     default: return cudaErrorInvalidValue;
     }

@@ -142,3 +142,25 @@ def test_fit_btf_reproduces_reference_pipeline(gpu_ctx, oracle_lib, golden):
     mean_ratio, within, worst = parity_stats(maps["rmse"], np.asarray(p["rmse"]))
     assert mean_ratio <= 1.01 and within >= 0.75, (mean_ratio, within, worst)
     b.close()
+
+
+@pytest.mark.parametrize("fmt,ds,ks,W,H", [
+    ("DFMF", 2, (48, 8, 16), 1, 1),      # whole groups of 8 components: the wide loads; one texel
+    ("DFMF", 2, (16, 24, 40), 63, 1),    # a texel short of a tile, half tiles of components
+    ("DFMF", 2, (15, 17, 1), 13, 5),     # one texel past a tile; components an element at a time
+    ("FMF1", 2, (8,), 32, 4),            # interleaved channels: rows of 3 K
+    ("FMF1", 2, (9,), 32, 2),
+    ("DFMF", 4, (16, 8, 32), 65, 1),
+    ("FMF1", 4, (31,), 16, 9)])
+def test_decode_tile_edges(gpu_ctx, oracle_lib, fmt, ds, ks, W, H):
+    """Bit for bit over the tiles' edges: 128 pairs (6561 leaves 33), 64 texels and
+    16 components; from a first texel inside the map too."""
+    planes, data = _ring_file(oracle_lib, fmt, ds, ks, W, H, seed=W + H + ds)
+    b = svf.Btf(gpu_ctx, data)
+    ref = oracle_lib.btf_decode(planes, fmt, W, H, 81, ds, 0, 0)
+    got = b.decode()
+    np.testing.assert_array_equal(got.view(np.uint32), ref.view(np.uint32))
+    T = W * H
+    np.testing.assert_array_equal(b.decode(first=T // 3, count=T - T // 3, sample_type=svf.SVF_SAMPLES_F16),
+                                  ref[T // 3:].astype(np.float16))
+    b.close()
