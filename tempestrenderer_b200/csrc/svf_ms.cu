@@ -141,10 +141,11 @@ __device__ __forceinline__ M3 cholesky(const M3& m)
 }
 
 // FloatIntelFastRand (functions.hh:214-218,249-252)
+__device__ __forceinline__ float lcg_value(unsigned s) { return (float)((s >> 16) & 0x7FFFu) / 32767.0f; }
 __device__ __forceinline__ float lcg(unsigned& s)
 {
     s = 214013u * s + 2531011u;
-    return (float)((s >> 16) & 0x7FFFu) / 32767.0f;
+    return lcg_value(s);
 }
 
 // SinCos_Tan (functions.hh:322-329), the reference's FastSinCos on the CPU
@@ -192,34 +193,121 @@ __device__ __forceinline__ float sggx_ndf(const NdfConst& k, V3 n)
     return k.num / (kPi * den * den);
 }
 
-// SGGXMicroFlakeSampleIncidentLight (ggx-models-impl.hh:554-570): a visible
-// normal of the distribution seen from `wo`, and wo reflected about it.  The
-// reference's GCC build evaluates the two FastFloatRand arguments of
-// UniformSampleSphere right to left: the second draws first.
-// cov: Matrix3::transformCovariance of the basis by stddev^2, fixed per evaluation.
-__device__ __forceinline__ V3 sample_incident(V3 wo, const M3& cov, unsigned& seed)
+// UniformSampleSphere (sampling3.hh:106-116) of the walk's next two numbers: the
+// reference's GCC build evaluates its two FastFloatRand arguments right to left, so
+// rb is the first drawn.
+__device__ __forceinline__ V3 sample_sphere(float rb, float ra)
 {
-    const float rb = lcg(seed);
-    const float ra = lcg(seed);
-    // UniformSampleSphere (sampling3.hh:106-116)
     float s, c;
     sincos_tan(2.0f * kPi * ra, &s, &c);
     const float ct = 2.0f * rb - 1.0f;
     const float st = sqrtf(1.0f - ct * ct);
-    const V3 u = v3(c * st, s * st, ct);
-    const M3 ob = basis_of(wo);
-    const M3 S = mmul(mmul(ob, cov), transpose(ob));
-    const V3 vn = transform(ob, normalize(rot_inverse(cholesky(S), u)));
+    return v3(c * st, s * st, ct);
+}
+
+// The numbers of an evaluation's walks.  Every evaluation of a launch draws from one
+// sequence (the seed is the launch's), so what the walks make of the numbers at a
+// position is the same in all of them: entry j of the table holds the sphere sample
+// of draws j and j + 1 and -log of draw j + 2, by the same operations as without it.
+// An event is then one 16-byte load, in place of three LCG steps and divisions, a
+// tangent, a square root and a logarithm.
+__device__ __forceinline__ void fill_walk_table(float4* tab, uint32_t entries, unsigned seed)
+{
+    for(uint32_t j = threadIdx.x; j < entries; j += blockDim.x)
+    {
+        unsigned mul_n = 1u, add_n = 0u, mul_1 = 214013u, add_1 = 2531011u;   // the LCG's j-th power
+        for(uint32_t n = j; n; n >>= 1)
+        {
+            if(n & 1)
+            {
+                add_n = add_n * mul_1 + add_1;
+                mul_n *= mul_1;
+            }
+            add_1 *= mul_1 + 1u;
+            mul_1 *= mul_1;
+        }
+        unsigned st = mul_n * seed + add_n;
+        const float rb = lcg_value(st);
+        const float ra = lcg(st);
+        const V3 u = sample_sphere(rb, ra);
+        tab[j] = make_float4(u.x, u.y, u.z, -logf(lcg(st)));
+    }
+    __syncthreads();
+}
+
+// The draws of `samples` walks of `depth` events, and so the table's entries.
+__host__ __device__ __forceinline__ uint64_t walk_draws(uint32_t samples, uint32_t depth)
+{
+    return 1 + (uint64_t)samples * (1 + 3 * (uint64_t)depth);
+}
+
+template <bool kTable>
+struct Draws
+{
+    const float4* tab;
+    uint32_t pos;     // draws so far (kTable)
+    unsigned state;   // the LCG's state (!kTable)
+
+    __device__ __forceinline__ float walk_log()
+    {
+        if constexpr(kTable)
+            return tab[pos++ - 1].w;
+        else
+            return -logf(lcg(state));
+    }
+    // an event's sphere sample and the -log of the number after it
+    __device__ __forceinline__ V3 event(float* log_next)
+    {
+        if constexpr(kTable)
+        {
+            const float4 e = tab[pos + 1];
+            pos += 3;
+            *log_next = e.w;
+            return v3(e.x, e.y, e.z);
+        }
+        else
+        {
+            const float rb = lcg(state);
+            const float ra = lcg(state);
+            const V3 u = sample_sphere(rb, ra);
+            *log_next = -logf(lcg(state));
+            return u;
+        }
+    }
+};
+
+// What SGGXMicroFlakeSampleIncidentLight (ggx-models-impl.hh:554-570) makes of its
+// direction alone: the frame and the Cholesky factor of the covariance seen in it.
+// cov: Matrix3::transformCovariance of the basis by stddev^2, fixed per evaluation.
+struct Seen
+{
+    M3 ob, chol;
+};
+__device__ __forceinline__ Seen seen_from(V3 wo, const M3& cov)
+{
+    Seen v;
+    v.ob = basis_of(wo);
+    v.chol = cholesky(mmul(mmul(v.ob, cov), transpose(v.ob)));
+    return v;
+}
+
+// The rest of it: a visible normal of the distribution seen from `wo`, and wo
+// reflected about it.
+__device__ __forceinline__ V3 sample_incident(V3 wo, const Seen& v, V3 u)
+{
+    const V3 vn = transform(v.ob, normalize(rot_inverse(v.chol, u)));
     return reflect(wo, vn);
 }
 
 // SGGXMicroFlakePseudoVolumeBRDF in the fitting frame (tangent x, binormal y,
 // normal z) for C spectrum channels; the walk continues while every channel's
 // throughput is above 1e-3.  The reference's Fresnel branch is compiled out
-// (USE_PSEUDO_VOLUME_FRESNEL is not defined).
-template <int C>
-__device__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const M3& b, float out_density, V3 wi, V3 wo,
-                              uint32_t depth, uint32_t samples, unsigned seed, float* out)
+// (USE_PSEUDO_VOLUME_FRESNEL is not defined).  Every walk starts at wo, so its first
+// event takes the frame of wo, worked out once.
+template <int C, bool kTable>
+__device__ __forceinline__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const M3& b,
+                                              float out_density, V3 wi, V3 wo, uint32_t depth, uint32_t samples,
+                                              unsigned seed, const float4* tab, float* out)
 {
     const float dot_inc = wi.z, dot_out = wo.z;
 #pragma unroll
@@ -230,6 +318,7 @@ __device__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const
     if(sd.x < 1e-6f || sd.y < 1e-6f)
         return;
     (void)lcg(seed);
+    Draws<kTable> draws{ tab, 1u, seed };
     const float in_density = projected_area(sd, b, wi);
     const V3 h = normalize(add(wo, wi));
     const float contrib = (float)samples / (out_density + in_density * dot_out / dot_inc);
@@ -237,44 +326,54 @@ __device__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const
     const NdfConst nk = ndf_const(sd, b);
     const M3 cov = covariance(b, mul(sd, sd));
     const float ndf = sggx_ndf(nk, h);
+    const Seen seen0 = seen_from(wo, cov);
     float rad[C], thr[C];
 #pragma unroll
     for(int c = 0; c < C; ++c)
         rad[c] = spec[c] * contrib * ndf * 2.0f * 0.25f;
-    for(uint32_t s = 0; s < samples; ++s)
-    {
+    V3 out_l;
+    float depth_in;
+    // a scattering event at out_l; whether the walk goes on
+    auto event = [&](const Seen& seen) {
+        float log_next;
+        const V3 u = draws.event(&log_next);
+        const V3 inc_l = sample_incident(out_l, seen, u);
+        const float dd = projected_area(sd, b, inc_l);
+        out_l = v3(-inc_l.x, -inc_l.y, -inc_l.z);
+        depth_in += (log_next / dd) * out_l.z;
+        if(depth_in < 0.0f)
+            return false;
+        const float ext = expf(-in_density * (depth_in / dot_inc));
+        if(ext < 1e-9f)
+            return false;
+        const float f = sggx_ndf(nk, normalize(add(out_l, wi))) * 2.0f / (4.0f * dd);
+        bool alive = true;   // (past the throughput test of the next event)
 #pragma unroll
         for(int c = 0; c < C; ++c)
-            thr[c] = spec[c];
-        V3 out_l = wo;
-        float dd = out_density;
-        float depth_in = (-logf(lcg(seed)) / dd) * dot_out;
-        for(uint32_t it = 0; it < depth; ++it)
         {
-            bool alive = true;
-#pragma unroll
-            for(int c = 0; c < C; ++c)
-                alive = alive && thr[c] > 1e-3f;
-            if(!alive)
-                break;
-            const V3 inc_l = sample_incident(out_l, cov, seed);
-            dd = projected_area(sd, b, inc_l);
-            out_l = v3(-inc_l.x, -inc_l.y, -inc_l.z);
-            depth_in += (-logf(lcg(seed)) / dd) * out_l.z;
-            if(depth_in < 0.0f)
-                break;
-            const float ext = expf(-in_density * (depth_in / dot_inc));
-            if(ext < 1e-9f)
-                break;
-            const float f = sggx_ndf(nk, normalize(add(out_l, wi))) * 2.0f / (4.0f * dd);
-#pragma unroll
-            for(int c = 0; c < C; ++c)
-            {
-                thr[c] *= spec[c];
-                rad[c] += ext * thr[c] * f;
-            }
+            thr[c] *= spec[c];
+            rad[c] += ext * thr[c] * f;
+            alive = alive && thr[c] > 1e-3f;
         }
-    }
+        return alive;
+    };
+    bool scatters = depth > 0;
+#pragma unroll
+    for(int c = 0; c < C; ++c)
+        scatters = scatters && spec[c] > 1e-3f;
+    if(scatters)
+        for(uint32_t s = 0; s < samples; ++s)
+        {
+#pragma unroll
+            for(int c = 0; c < C; ++c)
+                thr[c] = spec[c];
+            out_l = wo;
+            depth_in = (draws.walk_log() / out_density) * dot_out;
+            if(event(seen0))
+                for(uint32_t it = 1; it < depth; ++it)
+                    if(!event(seen_from(out_l, cov)))
+                        break;
+        }
     const float rcp = 1.0f / (float)samples;
 #pragma unroll
     for(int c = 0; c < C; ++c)
@@ -307,10 +406,13 @@ __device__ __forceinline__ M3 euler_matrix(const float* e)
     return quat_matrix(q);
 }
 
+constexpr uint32_t kFitWalks = 256;
+
 // BRDFEvaluator::operator() with BounceCount = depth (svbrdf-lsq-fitting-
 // internal.hh:91-153): parameters handed over as doubles and rounded to float,
 // 256 walks from LCG seed 0 (the evaluator's texture coordinate is 0).
-__device__ float evaluator_ms(const double* pd, V3 wi, V3 wo, uint32_t depth)
+template <bool kTable>
+__device__ float evaluator_ms(const double* pd, V3 wi, V3 wo, uint32_t depth, const float4* tab)
 {
     float p[7];
 #pragma unroll
@@ -321,7 +423,7 @@ __device__ float evaluator_ms(const double* pd, V3 wi, V3 wo, uint32_t depth)
     const float ks = p[2] > 0.0f ? p[2] : 0.0f;
     const float kd = p[3] > 0.0f ? p[3] : 0.0f;
     float r;
-    pseudo_volume<1>(&ks, &kd, sd, b, projected_area(sd, b, wo), wi, wo, depth, 256u, 0u, &r);
+    pseudo_volume<1, kTable>(&ks, &kd, sd, b, projected_area(sd, b, wo), wi, wo, depth, kFitWalks, 0u, tab, &r);
     return r;
 }
 
@@ -330,12 +432,34 @@ __device__ __forceinline__ V3 direction(const float* geo, uint32_t L, uint32_t d
     return v3(geo[d], geo[L + d], geo[2 * L + d]);
 }
 
+constexpr int kMsThreads = 256;
+
+// Shared memory of the walk table; 0 where there is none: past 96 KB two CTAs no longer
+// fit on an SM (256 walks of 7 events take 90 KB).
+size_t walk_table_bytes(uint32_t samples, uint32_t depth)
+{
+    const uint64_t bytes = sizeof(float4) * walk_draws(samples, depth);
+    return bytes <= 96 * 1024 ? (size_t)bytes : 0;
+}
+
+template <typename Kernel>
+cudaError_t allow_smem(Kernel* kernel, size_t bytes)
+{
+    if(bytes <= 48 * 1024)
+        return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(96 * 1024));
+}
+
 } // namespace
 
 // ---- rendering ----------------------------------------------------------------------
 
-__global__ void __launch_bounds__(128) ms_render_kernel(MsRenderArgs a)
+template <bool kTable>
+__global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
 {
+    extern __shared__ float4 walk_table[];
+    if constexpr(kTable)
+        fill_walk_table(walk_table, (uint32_t)walk_draws(a.samples, a.bounces), a.seed);
     const uint64_t N = (uint64_t)a.L * a.L;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= a.count * N)
@@ -364,7 +488,8 @@ __global__ void __launch_bounds__(128) ms_render_kernel(MsRenderArgs a)
     const M3 b = quat_matrix(q);
     const V3 wi = direction(a.geo, a.L, light), wo = direction(a.geo, a.L, view);
     float f[3];
-    pseudo_volume<3>(ks, kd, sd, b, projected_area(sd, b, wo), wi, wo, a.bounces, a.samples, a.seed, f);
+    pseudo_volume<3, kTable>(ks, kd, sd, b, projected_area(sd, b, wo), wi, wo, a.bounces, a.samples, a.seed, walk_table,
+                             f);
     const uint64_t o = i * 3;
 #pragma unroll
     for(int c = 0; c < 3; ++c)
@@ -381,10 +506,19 @@ cudaError_t launch_ms_render(const MsRenderArgs& a, cudaStream_t stream)
     const uint64_t n = a.count * (uint64_t)a.L * a.L;
     if(n == 0)
         return cudaSuccess;
-    const uint64_t blocks = (n + 127) / 128;
+    const uint64_t blocks = (n + kMsThreads - 1) / kMsThreads;
     if(blocks > 0x7fffffffull)
         return cudaErrorInvalidValue;
-    ms_render_kernel<<<(unsigned)blocks, 128, 0, stream>>>(a);
+    const size_t smem = walk_table_bytes(a.samples, a.bounces);
+    if(smem == 0)
+        ms_render_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(a);
+    else
+    {
+        const cudaError_t e = allow_smem(ms_render_kernel<true>, smem);
+        if(e != cudaSuccess)
+            return e;
+        ms_render_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(a);
+    }
     return cudaGetLastError();
 }
 
@@ -420,13 +554,19 @@ __device__ __forceinline__ void fd_params(const MsTexel& s, int e, double* p)
 } // namespace
 
 // count: the list's length, or (dcount non-null) at most this many, *dcount
-__global__ void __launch_bounds__(128) ms_eval_kernel(MsFitArgs a, uint32_t mode, uint32_t count,
-                                                      const uint32_t* dcount)
+template <bool kTable>
+__global__ void __launch_bounds__(kMsThreads) ms_eval_kernel(MsFitArgs a, uint32_t mode, uint32_t count,
+                                                             const uint32_t* dcount)
 {
+    extern __shared__ float4 walk_table[];
     if(dcount)
         count = min(count, *dcount);
     const uint64_t N = (uint64_t)a.L * a.L;
     const uint64_t per = mode == kMsEvalJacobian ? N * kMsEvals : N;
+    if((uint64_t)blockIdx.x * blockDim.x >= (uint64_t)count * per)
+        return;
+    if constexpr(kTable)
+        fill_walk_table(walk_table, (uint32_t)walk_draws(kFitWalks, a.bounces), 0u);
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= (uint64_t)count * per)
         return;
@@ -439,10 +579,10 @@ __global__ void __launch_bounds__(128) ms_eval_kernel(MsFitArgs a, uint32_t mode
     {
         double p[7];
         fd_params(s, (int)(r % kMsEvals), p);
-        a.fev[(uint64_t)t * N * kMsEvals + r] = -evaluator_ms(p, wi, wo, a.bounces);
+        a.fev[(uint64_t)t * N * kMsEvals + r] = -evaluator_ms<kTable>(p, wi, wo, a.bounces, walk_table);
         return;
     }
-    const float f = evaluator_ms(mode == kMsEvalTrial ? s.tmp : s.p, wi, wo, a.bounces);
+    const float f = evaluator_ms<kTable>(mode == kMsEvalTrial ? s.tmp : s.p, wi, wo, a.bounces, walk_table);
     a.res[(uint64_t)t * N + idx] = a.lum[t * a.lum_stride + idx] - f;
 }
 
@@ -787,11 +927,21 @@ cudaError_t launch_ms_eval(const MsFitArgs& a, uint32_t mode, uint32_t count, co
         return cudaSuccess;
     const uint64_t N = (uint64_t)a.L * a.L;
     const uint64_t n = (uint64_t)count * N * (mode == kMsEvalJacobian ? kMsEvals : 1);
-    const uint64_t blocks = (n + 127) / 128;
+    const uint64_t blocks = (n + kMsThreads - 1) / kMsThreads;
     if(blocks > 0x7fffffffull)
         return cudaErrorInvalidValue;
-    ms_eval_kernel<<<(unsigned)blocks, 128, 0, stream>>>(a, mode, count, dcount);
-    cudaError_t e = cudaGetLastError();
+    const size_t smem = walk_table_bytes(kFitWalks, a.bounces);
+    cudaError_t e = cudaSuccess;
+    if(smem == 0)
+        ms_eval_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(a, mode, count, dcount);
+    else
+    {
+        e = allow_smem(ms_eval_kernel<true>, smem);
+        if(e != cudaSuccess)
+            return e;
+        ms_eval_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(a, mode, count, dcount);
+    }
+    e = cudaGetLastError();
     if(e != cudaSuccess)
         return e;
     ms_reduce_kernel<<<count, 256, 0, stream>>>(a, mode, dcount);
