@@ -190,6 +190,7 @@ struct svf_ctx
     svfh::DevBuf lum, lum_hi, lum_lo, avg, ndf, ndf_tex, init, out, rmse, stats, counter, error, samples, samples2,
         maps_buf, scratch, rgb16, init_rgb, mlp_x, mlp_h1, mlp_h2, mlp_y, fb_idx, fb_lum, fb_hi, fb_lo, fb_ndf,
         fb_small,
+        ms_walks /* svf_render_btf_ms: the views' walks, kept between calls (at most kMsWalkBytes) */,
         btf_decoded /* svf_fit_btf: the decoded chunk, kept between calls */;
     svfh::PinnedBuf pinned;
 };

@@ -9,7 +9,8 @@
 // the parallelism is over texels, direction pairs and (for the Jacobian) the
 // 14 perturbed parameter vectors of a pair.
 //
-//   ms_render_kernel    the BTF of SVBRDF maps with this BRDF (RGB)
+//   ms_render_kernel    the BTF of SVBRDF maps with this BRDF (RGB); of many pairs
+//                       ms_walk_kernel, ms_lookup_kernel and ms_rest_kernel
 //   ms_eval_kernel      residuals of the luminance fit, or the 14 central-
 //                       difference evaluations of a pair's Jacobian row
 //   ms_reduce_kernel    a texel's residual sum, or J^T J and J^T r (FP64, fixed order)
@@ -23,6 +24,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "../../include/svf.h"
 #include "svf_internal.h"
@@ -299,85 +302,135 @@ __device__ __forceinline__ V3 sample_incident(V3 wo, const Seen& v, V3 u)
     return reflect(wo, vn);
 }
 
-// SGGXMicroFlakePseudoVolumeBRDF in the fitting frame (tangent x, binormal y,
-// normal z) for C spectrum channels; the walk continues while every channel's
-// throughput is above 1e-3.  The reference's Fresnel branch is compiled out
-// (USE_PSEUDO_VOLUME_FRESNEL is not defined).  Every walk starts at wo, so its first
-// event takes the frame of wo, worked out once.
-template <int C, bool kTable>
-__device__ __forceinline__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const M3& b,
-                                              float out_density, V3 wi, V3 wo, uint32_t depth, uint32_t samples,
-                                              unsigned seed, const float4* tab, float* out)
+// The next scattering event of a walk that looks along out_l at depth_in: the
+// direction it leaves in, the projected area along it and the depth where the next
+// event lies.
+template <bool kTable>
+__device__ __forceinline__ void scatter(Draws<kTable>& draws, const Seen& seen, V3 sd, const M3& b, V3& out_l,
+                                        float& depth_in, float& dd)
 {
-    const float dot_inc = wi.z, dot_out = wo.z;
+    float log_next;
+    const V3 u = draws.event(&log_next);
+    const V3 inc_l = sample_incident(out_l, seen, u);
+    dd = projected_area(sd, b, inc_l);
+    out_l = v3(-inc_l.x, -inc_l.y, -inc_l.z);
+    depth_in += (log_next / dd) * out_l.z;
+}
+
+// SGGXMicroFlakePseudoVolumeBRDF in the fitting frame (tangent x, binormal y,
+// normal z) for C spectrum channels; a walk continues while every channel's
+// throughput is above 1e-3.  The reference's Fresnel branch is compiled out
+// (USE_PSEUDO_VOLUME_FRESNEL is not defined).  One (light, view) pair's evaluation:
+template <int C>
+struct PairEval
+{
+    V3 wi, wo;
+    float in_density, rad[C];
+    NdfConst nk;
+
+    // false: the BRDF is zero
+    __device__ __forceinline__ static bool lit(V3 sd, V3 wi, V3 wo)
+    {
+        return !(wo.z < 0.0f || wi.z < 0.0f) && !(sd.x < 1e-6f || sd.y < 1e-6f);
+    }
+    // the single-scattering term
+    __device__ __forceinline__ void start(const float* spec, V3 sd, const M3& b, float out_density, V3 wi_, V3 wo_,
+                                          uint32_t samples)
+    {
+        wi = wi_;
+        wo = wo_;
+        const float dot_inc = wi.z, dot_out = wo.z;
+        in_density = projected_area(sd, b, wi);
+        const V3 h = normalize(add(wo, wi));
+        const float contrib = (float)samples / (out_density + in_density * dot_out / dot_inc);
+        // what the evaluation's parameters fix, computed once (the reference recomputes it per call)
+        nk = ndf_const(sd, b);
+        const float ndf = sggx_ndf(nk, h);
 #pragma unroll
-    for(int c = 0; c < C; ++c)
-        out[c] = 0.0f;
-    if(dot_out < 0.0f || dot_inc < 0.0f)
-        return;
-    if(sd.x < 1e-6f || sd.y < 1e-6f)
-        return;
-    (void)lcg(seed);
-    Draws<kTable> draws{ tab, 1u, seed };
-    const float in_density = projected_area(sd, b, wi);
-    const V3 h = normalize(add(wo, wi));
-    const float contrib = (float)samples / (out_density + in_density * dot_out / dot_inc);
-    // what the evaluation's parameters fix, computed once (the reference recomputes it per call)
-    const NdfConst nk = ndf_const(sd, b);
-    const M3 cov = covariance(b, mul(sd, sd));
-    const float ndf = sggx_ndf(nk, h);
-    const Seen seen0 = seen_from(wo, cov);
-    float rad[C], thr[C];
-#pragma unroll
-    for(int c = 0; c < C; ++c)
-        rad[c] = spec[c] * contrib * ndf * 2.0f * 0.25f;
-    V3 out_l;
-    float depth_in;
-    // a scattering event at out_l; whether the walk goes on
-    auto event = [&](const Seen& seen) {
-        float log_next;
-        const V3 u = draws.event(&log_next);
-        const V3 inc_l = sample_incident(out_l, seen, u);
-        const float dd = projected_area(sd, b, inc_l);
-        out_l = v3(-inc_l.x, -inc_l.y, -inc_l.z);
-        depth_in += (log_next / dd) * out_l.z;
-        if(depth_in < 0.0f)
-            return false;
-        const float ext = expf(-in_density * (depth_in / dot_inc));
+        for(int c = 0; c < C; ++c)
+            rad[c] = spec[c] * contrib * ndf * 2.0f * 0.25f;
+    }
+    // the light from wi that an event at depth_in sends along the walk; dd4: 4 times
+    // the projected area along it.  Whether it is visible there (the walk ends else).
+    __device__ __forceinline__ bool event(const float* spec, V3 out_l, float depth_in, float dd4, float* thr)
+    {
+        const float ext = expf(-in_density * (depth_in / wi.z));
         if(ext < 1e-9f)
             return false;
-        const float f = sggx_ndf(nk, normalize(add(out_l, wi))) * 2.0f / (4.0f * dd);
-        bool alive = true;   // (past the throughput test of the next event)
+        const float f = sggx_ndf(nk, normalize(add(out_l, wi))) * 2.0f / dd4;
 #pragma unroll
         for(int c = 0; c < C; ++c)
         {
             thr[c] *= spec[c];
             rad[c] += ext * thr[c] * f;
-            alive = alive && thr[c] > 1e-3f;
         }
-        return alive;
-    };
-    bool scatters = depth > 0;
+        return true;
+    }
+    __device__ __forceinline__ static bool alive(const float* thr)
+    {
+        bool on = true;
 #pragma unroll
-    for(int c = 0; c < C; ++c)
-        scatters = scatters && spec[c] > 1e-3f;
-    if(scatters)
-        for(uint32_t s = 0; s < samples; ++s)
+        for(int c = 0; c < C; ++c)
+            on = on && thr[c] > 1e-3f;
+        return on;
+    }
+    // walks first .. samples - 1
+    template <bool kTable>
+    __device__ __forceinline__ void walks(const float* spec, V3 sd, const M3& b, float out_density, uint32_t depth,
+                                          uint32_t first, uint32_t samples, Draws<kTable> draws)
+    {
+        if(depth == 0 || !alive(spec))
+            return;
+        const M3 cov = covariance(b, mul(sd, sd));
+        const Seen seen0 = seen_from(wo, cov);   // every walk starts along wo
+        float thr[C];
+        for(uint32_t s = first; s < samples; ++s)
         {
 #pragma unroll
             for(int c = 0; c < C; ++c)
                 thr[c] = spec[c];
-            out_l = wo;
-            depth_in = (draws.walk_log() / out_density) * dot_out;
-            if(event(seen0))
-                for(uint32_t it = 1; it < depth; ++it)
-                    if(!event(seen_from(out_l, cov)))
-                        break;
+            V3 out_l = wo;
+            float depth_in = (draws.walk_log() / out_density) * wo.z, dd;
+            scatter(draws, seen0, sd, b, out_l, depth_in, dd);
+            for(uint32_t it = 1;; ++it)
+            {
+                if(depth_in < 0.0f || !event(spec, out_l, depth_in, 4.0f * dd, thr) || it == depth || !alive(thr))
+                    break;
+                scatter(draws, seen_from(out_l, cov), sd, b, out_l, depth_in, dd);
+            }
         }
-    const float rcp = 1.0f / (float)samples;
+    }
+    __device__ __forceinline__ void finish(const float* diff, uint32_t samples, float* out) const
+    {
+        const float rcp = 1.0f / (float)samples;
+#pragma unroll
+        for(int c = 0; c < C; ++c)
+            out[c] = rad[c] * rcp + diff[c] * wi.z * (1.0f / kPi);
+    }
+};
+
+// The sequence's first draw is dropped.
+template <bool kTable>
+__device__ __forceinline__ Draws<kTable> first_draws(unsigned seed, const float4* tab)
+{
+    (void)lcg(seed);
+    return Draws<kTable>{ tab, 1u, seed };
+}
+
+template <int C, bool kTable>
+__device__ __forceinline__ void pseudo_volume(const float* spec, const float* diff, V3 sd, const M3& b,
+                                              float out_density, V3 wi, V3 wo, uint32_t depth, uint32_t samples,
+                                              unsigned seed, const float4* tab, float* out)
+{
 #pragma unroll
     for(int c = 0; c < C; ++c)
-        out[c] = rad[c] * rcp + diff[c] * dot_inc * (1.0f / kPi);
+        out[c] = 0.0f;
+    if(!PairEval<C>::lit(sd, wi, wo))
+        return;
+    PairEval<C> e;
+    e.start(spec, sd, b, out_density, wi, wo, samples);
+    e.walks(spec, sd, b, out_density, depth, 0, samples, first_draws<kTable>(seed, tab));
+    e.finish(diff, samples, out);
 }
 
 // ToQuaternion(euler) (quaternion.hh:82-94) with the reference's FastSinCos,
@@ -432,7 +485,9 @@ __device__ __forceinline__ V3 direction(const float* geo, uint32_t L, uint32_t d
     return v3(geo[d], geo[L + d], geo[2 * L + d]);
 }
 
-constexpr int kMsThreads = 256;
+constexpr int kMsThreads = 256, kWalkThreads = 64;
+constexpr int kRestThreads = 128;
+constexpr uint64_t kRestBlocks = 5 * 148;   // (as many as are resident)
 
 // Shared memory of the walk table; 0 where there is none: past 96 KB two CTAs no longer
 // fit on an SM (256 walks of 7 events take 90 KB).
@@ -454,19 +509,19 @@ cudaError_t allow_smem(Kernel* kernel, size_t bytes)
 
 // ---- rendering ----------------------------------------------------------------------
 
-template <bool kTable>
-__global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
+namespace
 {
-    extern __shared__ float4 walk_table[];
-    if constexpr(kTable)
-        fill_walk_table(walk_table, (uint32_t)walk_draws(a.samples, a.bounces), a.seed);
-    const uint64_t N = (uint64_t)a.L * a.L;
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= a.count * N)
-        return;
-    const uint64_t t = i / N;
-    const uint32_t lv = (uint32_t)(i % N);
-    const uint32_t view = lv / a.L, light = lv % a.L;
+
+// A texel's material from the maps.
+struct MsMaterial
+{
+    V3 sd;
+    float kd[3], ks[3];
+    M3 b;
+};
+__device__ __forceinline__ MsMaterial ms_material(const MsRenderArgs& a, uint64_t t)
+{
+    MsMaterial m;
     float sx = a.sigma[a.sigma_channels * t], sy = a.sigma[a.sigma_channels * t + 1];
     if(a.sigma_channels == 3)
     {
@@ -474,22 +529,24 @@ __global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
         sx = sx / sz;
         sy = sy / sz;
     }
-    const V3 sd = v3(sx > 0.0f ? sx : 0.0f, sy > 0.0f ? sy : 0.0f, 1.0f);
-    float q[4], kd[3], ks[3];
+    m.sd = v3(sx > 0.0f ? sx : 0.0f, sy > 0.0f ? sy : 0.0f, 1.0f);
+    float q[4];
 #pragma unroll
     for(int k = 0; k < 4; ++k)
         q[k] = a.basis[4 * t + k];
 #pragma unroll
     for(int c = 0; c < 3; ++c)
     {
-        kd[c] = fmaxf(a.diffuse[3 * t + c], 0.0f);
-        ks[c] = fmaxf(a.specular[3 * t + c], 0.0f);
+        m.kd[c] = fmaxf(a.diffuse[3 * t + c], 0.0f);
+        m.ks[c] = fmaxf(a.specular[3 * t + c], 0.0f);
     }
-    const M3 b = quat_matrix(q);
-    const V3 wi = direction(a.geo, a.L, light), wo = direction(a.geo, a.L, view);
-    float f[3];
-    pseudo_volume<3, kTable>(ks, kd, sd, b, projected_area(sd, b, wo), wi, wo, a.bounces, a.samples, a.seed, walk_table,
-                             f);
+    m.b = quat_matrix(q);
+    return m;
+}
+
+// A pair's three values in the output's sample type.
+__device__ __forceinline__ void store_pair(const MsRenderArgs& a, uint64_t i, const float* f)
+{
     const uint64_t o = i * 3;
 #pragma unroll
     for(int c = 0; c < 3; ++c)
@@ -501,25 +558,235 @@ __global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
     }
 }
 
-cudaError_t launch_ms_render(const MsRenderArgs& a, cudaStream_t stream)
+} // namespace
+
+// The walks of an evaluation are those of its view: the light enters only in what an
+// event sends along and in the test whether it still sees it (the walk ends there, and
+// the evaluation's later numbers are others than its view's).  So the views' walks are
+// worked out once (ms_walk_kernel) and the pairs look their events up
+// (ms_lookup_kernel); a pair that loses sight of an event that its view's walk goes on
+// from leaves its sums in a list, and the rest of its walks are its own
+// (ms_rest_kernel).  16 x 16 texels of ring-81, 256 walks of two events: 0.31 + 4.0 +
+// 1.1 ms, where every pair walking by itself (ms_render_kernel) takes 11.6, and 16.1
+// without the table of draws.  Finishing the lost pairs in the lookup takes 9.9: a few
+// lanes of a warp then walk for all, on half as many warps.
+struct MsRest
 {
-    const uint64_t n = a.count * (uint64_t)a.L * a.L;
-    if(n == 0)
-        return cudaSuccess;
-    const uint64_t blocks = (n + kMsThreads - 1) / kMsThreads;
-    if(blocks > 0x7fffffffull)
-        return cudaErrorInvalidValue;
-    const size_t smem = walk_table_bytes(a.samples, a.bounces);
-    if(smem == 0)
-        ms_render_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(a);
-    else
+    uint64_t i;        // the pair
+    uint32_t s, pos;   // its next walk, the draws before it
+    float rad[3];
+};
+
+struct MsWalks
+{
+    float4* ev;      // [texel][view][walk][event]: direction, depth
+    float* dd4;      // 4 times the projected area along it
+    MsRest* rest;    // room for every pair
+    uint32_t* lost;  // their number
+};
+
+// One thread per (texel, view): the walks as they go on while no light loses sight of
+// an event; one that leaves the volume ends with a record of negative depth.
+__global__ void __launch_bounds__(kWalkThreads) ms_walk_kernel(MsRenderArgs a, MsWalks w)
+{
+    extern __shared__ float4 walk_table[];
+    fill_walk_table(walk_table, (uint32_t)walk_draws(a.samples, a.bounces), a.seed);
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i == 0)
+        *w.lost = 0;
+    if(i >= a.count * a.L)
+        return;
+    const MsMaterial m = ms_material(a, i / a.L);
+    const V3 wo = direction(a.geo, a.L, (uint32_t)(i % a.L));
+    if(!PairEval<3>::lit(m.sd, wo, wo) || !PairEval<3>::alive(m.ks))
+        return;
+    const float out_density = projected_area(m.sd, m.b, wo);
+    const M3 cov = covariance(m.b, mul(m.sd, m.sd));
+    const Seen seen0 = seen_from(wo, cov);
+    Draws<true> draws = first_draws<true>(a.seed, walk_table);
+    for(uint32_t s = 0; s < a.samples; ++s)
     {
-        const cudaError_t e = allow_smem(ms_render_kernel<true>, smem);
-        if(e != cudaSuccess)
-            return e;
-        ms_render_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(a);
+        float thr[3] = { m.ks[0], m.ks[1], m.ks[2] };
+        V3 out_l = wo;
+        float depth_in = (draws.walk_log() / out_density) * wo.z, dd;
+        scatter(draws, seen0, m.sd, m.b, out_l, depth_in, dd);
+        for(uint32_t e = 0;;)
+        {
+            const uint64_t r = (i * a.samples + s) * a.bounces + e;
+            w.ev[r] = make_float4(out_l.x, out_l.y, out_l.z, depth_in);
+            w.dd4[r] = 4.0f * dd;
+#pragma unroll
+            for(int c = 0; c < 3; ++c)
+                thr[c] *= m.ks[c];
+            if(depth_in < 0.0f || ++e == a.bounces || !PairEval<3>::alive(thr))
+                break;
+            scatter(draws, seen_from(out_l, cov), m.sd, m.b, out_l, depth_in, dd);
+        }
     }
-    return cudaGetLastError();
+}
+
+// One thread per (texel, view, light), bound by the issue of the events' arithmetic
+// (three divisions, a reciprocal, a square root and an exponential, correctly rounded).
+__global__ void __launch_bounds__(kMsThreads, 4) ms_lookup_kernel(MsRenderArgs a, MsWalks w)
+{
+    const uint64_t N = (uint64_t)a.L * a.L;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= a.count * N)
+        return;
+    const uint64_t t = i / N;
+    const uint32_t lv = (uint32_t)(i % N);
+    const uint32_t view = lv / a.L, light = lv % a.L;
+    const MsMaterial m = ms_material(a, t);
+    const V3 wi = direction(a.geo, a.L, light), wo = direction(a.geo, a.L, view);
+    float f[3] = { 0.0f, 0.0f, 0.0f };
+    if(PairEval<3>::lit(m.sd, wi, wo))
+    {
+        PairEval<3> p;
+        p.start(m.ks, m.sd, m.b, projected_area(m.sd, m.b, wo), wi, wo, a.samples);
+        const uint64_t first = (t * a.L + view) * a.samples * a.bounces;
+        const float4* ev = w.ev + first;
+        const float* dd4 = w.dd4 + first;
+        uint32_t pos = 1;
+        if(PairEval<3>::alive(m.ks))
+            for(uint32_t s = 0; s < a.samples; ++s, ev += a.bounces, dd4 += a.bounces)
+            {
+                float thr[3] = { m.ks[0], m.ks[1], m.ks[2] };
+                ++pos;
+                bool lost = false;
+                for(uint32_t e = 0;;)
+                {
+                    const float4 x = ev[e];
+                    pos += 3;
+                    if(x.w < 0.0f)
+                        break;
+                    const bool seen = p.event(m.ks, v3(x.x, x.y, x.z), x.w, dd4[e], thr);
+                    if(!seen)   // (the view's throughput after the event)
+#pragma unroll
+                        for(int c = 0; c < 3; ++c)
+                            thr[c] *= m.ks[c];
+                    if(++e == a.bounces || !PairEval<3>::alive(thr))
+                        break;
+                    if(!seen)
+                    {
+                        lost = true;
+                        break;
+                    }
+                }
+                if(lost && s + 1 < a.samples)
+                {
+                    w.rest[atomicAdd(w.lost, 1u)] = MsRest{ i, s + 1, pos, { p.rad[0], p.rad[1], p.rad[2] } };
+                    return;
+                }
+            }
+        p.finish(m.kd, a.samples, f);
+    }
+    store_pair(a, i, f);
+}
+
+__global__ void __launch_bounds__(kRestThreads) ms_rest_kernel(MsRenderArgs a, MsWalks w)
+{
+    extern __shared__ float4 walk_table[];
+    const uint32_t lost = *w.lost;
+    if((uint64_t)blockIdx.x * blockDim.x >= lost)
+        return;
+    fill_walk_table(walk_table, (uint32_t)walk_draws(a.samples, a.bounces), a.seed);
+    const uint64_t N = (uint64_t)a.L * a.L;
+    for(uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < lost; k += (uint64_t)gridDim.x * blockDim.x)
+    {
+        const MsRest r = w.rest[k];
+        const uint32_t lv = (uint32_t)(r.i % N);
+        const MsMaterial m = ms_material(a, r.i / N);
+        const V3 wi = direction(a.geo, a.L, lv % a.L), wo = direction(a.geo, a.L, lv / a.L);
+        PairEval<3> p;
+        const float out_density = projected_area(m.sd, m.b, wo);
+        p.start(m.ks, m.sd, m.b, out_density, wi, wo, a.samples);
+#pragma unroll
+        for(int c = 0; c < 3; ++c)
+            p.rad[c] = r.rad[c];
+        p.walks(m.ks, m.sd, m.b, out_density, a.bounces, r.s, a.samples, Draws<true>{ walk_table, r.pos, 0u });
+        float f[3];
+        p.finish(m.kd, a.samples, f);
+        store_pair(a, r.i, f);
+    }
+}
+
+// One thread per (texel, view, light), every pair with walks of its own: of few pairs,
+// and where the views' walks have no room.
+template <bool kTable>
+__global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
+{
+    extern __shared__ float4 walk_table[];
+    if constexpr(kTable)
+        fill_walk_table(walk_table, (uint32_t)walk_draws(a.samples, a.bounces), a.seed);
+    const uint64_t N = (uint64_t)a.L * a.L;
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if(i >= a.count * N)
+        return;
+    const uint32_t lv = (uint32_t)(i % N);
+    const MsMaterial m = ms_material(a, i / N);
+    const V3 wi = direction(a.geo, a.L, lv % a.L), wo = direction(a.geo, a.L, lv / a.L);
+    float f[3];
+    pseudo_volume<3, kTable>(m.ks, m.kd, m.sd, m.b, projected_area(m.sd, m.b, wo), wi, wo, a.bounces, a.samples, a.seed,
+                             walk_table, f);
+    store_pair(a, i, f);
+}
+
+uint64_t ms_walk_bytes(uint32_t L, uint32_t samples, uint32_t bounces)
+{
+    if(bounces == 0 || walk_table_bytes(samples, bounces) == 0)
+        return 0;
+    return (uint64_t)L * samples * bounces * (sizeof(float4) + sizeof(float)) + (uint64_t)L * L * sizeof(MsRest);
+}
+
+cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk_texels, cudaStream_t stream)
+{
+    const uint64_t N = (uint64_t)all.L * all.L;
+    if(all.count * N == 0)
+        return cudaSuccess;
+    const size_t smem = walk_table_bytes(all.samples, all.bounces);
+    cudaError_t e = cudaSuccess;
+    auto blocks_of = [](uint64_t n, int threads) { return (n + threads - 1) / threads; };
+    if(!walks)
+    {
+        const uint64_t blocks = blocks_of(all.count * N, kMsThreads);
+        if(blocks > 0x7fffffffull)
+            return cudaErrorInvalidValue;
+        if(smem == 0)
+            ms_render_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(all);
+        else if((e = allow_smem(ms_render_kernel<true>, smem)) != cudaSuccess)
+            return e;
+        else
+            ms_render_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(all);
+        return cudaGetLastError();
+    }
+    if((e = allow_smem(ms_walk_kernel, smem)) != cudaSuccess || (e = allow_smem(ms_rest_kernel, smem)) != cudaSuccess)
+        return e;
+    MsWalks w;
+    const uint64_t events = walk_texels * all.L * all.samples * all.bounces;
+    w.lost = static_cast<uint32_t*>(walks);
+    w.ev = reinterpret_cast<float4*>(w.lost + kMsWalkHeader / sizeof(uint32_t));
+    w.rest = reinterpret_cast<MsRest*>(w.ev + events);
+    w.dd4 = reinterpret_cast<float*>(w.rest + walk_texels * N);
+    for(uint64_t t0 = 0; t0 < all.count; t0 += walk_texels)
+    {
+        MsRenderArgs a = all;
+        a.count = all.count - t0 < walk_texels ? all.count - t0 : walk_texels;
+        a.diffuse += 3 * t0;
+        a.specular += 3 * t0;
+        a.sigma += a.sigma_channels * t0;
+        a.basis += 4 * t0;
+        a.out = static_cast<char*>(a.out) + t0 * N * 3 * (a.sample_type == SVF_SAMPLES_F16 ? 2 : 4);
+        const uint64_t pairs = blocks_of(a.count * N, kMsThreads), views = blocks_of(a.count * a.L, kWalkThreads);
+        if(pairs > 0x7fffffffull || views > 0x7fffffffull || a.count * N > 0xffffffffull)
+            return cudaErrorInvalidValue;
+        ms_walk_kernel<<<(unsigned)views, kWalkThreads, smem, stream>>>(a, w);
+        ms_lookup_kernel<<<(unsigned)pairs, kMsThreads, 0, stream>>>(a, w);
+        const uint64_t rest = std::min(blocks_of(a.count * N, kRestThreads), kRestBlocks);
+        ms_rest_kernel<<<(unsigned)rest, kRestThreads, smem, stream>>>(a, w);
+        if((e = cudaGetLastError()) != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
 }
 
 // ---- the multi-scattering LM fit ------------------------------------------------------

@@ -175,3 +175,30 @@ def test_invalid_option_combinations(gpu_ctx, kw):
     with pytest.raises(svf.SvfError) as e:
         gpu_ctx.lsq_fit_batch(lp, lum, init, svf.options(multi_scattering=2, **kw))
     assert e.value.status == svf.SVF_EINVAL
+
+
+@pytest.mark.parametrize("T,bounces,samples,seed,half", [
+    (90, 1, 256, 0, False), (90, 2, 256, 7, True), (90, 5, 31, 1, False),
+    (600, 3, 256, 0, False),    # more texels than the walks' memory holds at a time
+    (80, 8, 256, 0, False),     # too deep for the table of draws
+    (80, 2, 2, 3, False), (80, 0, 16, 0, False)])
+def test_shared_walks_equal_own_walks(gpu_ctx, ms, T, bounces, samples, seed, half):
+    """A call of many pairs shares the views' walks, one of few lets every pair walk by
+    itself (at most 512 pairs an SM): bit for bit the same samples."""
+    rng = np.random.default_rng(T + bounces)
+    q = rng.standard_normal((T, 4)).astype(np.float32)
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    sigma = (0.05 + 0.9 * rng.random((T, 2))).astype(np.float32)
+    sigma[5] = 0.0                                      # no surface: zeros
+    diffuse = (0.3 * rng.random((T, 3))).astype(np.float32)
+    specular = (0.02 + 1.5 * rng.random((T, 3))).astype(np.float32)
+    specular[7, 1] = 5e-4                               # no walk; three texels die after one event
+    specular[8:11] = 0.02
+    typ = svf.SVF_SAMPLES_F16 if half else svf.SVF_SAMPLES_F32
+    lp = ms["fib32"]
+    got = gpu_ctx.render_btf_ms(lp, diffuse, specular, sigma, q, bounces, samples=samples, seed=seed, sample_type=typ)
+    own = np.concatenate([gpu_ctx.render_btf_ms(lp, diffuse[t:t + 40], specular[t:t + 40], sigma[t:t + 40],
+                                                q[t:t + 40], bounces, samples=samples, seed=seed, sample_type=typ)
+                          for t in range(0, T, 40)])
+    word = np.uint16 if half else np.uint32
+    np.testing.assert_array_equal(got.view(word), own.view(word))
