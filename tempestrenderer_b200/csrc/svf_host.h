@@ -191,7 +191,8 @@ struct svf_ctx
         maps_buf, scratch, rgb16, init_rgb, mlp_x, mlp_h1, mlp_h2, mlp_y, fb_idx, fb_lum, fb_hi, fb_lo, fb_ndf,
         fb_small,
         ms_walks /* svf_render_btf_ms: the views' walks, kept between calls (at most kMsWalkBytes) */,
-        btf_decoded /* svf_fit_btf: the decoded chunk, kept between calls */;
+        btf_decoded /* svf_fit_btf, svf_error_maps: the decoded chunk, kept between calls */,
+        btf_maps /* svf_error_maps, svf_render_btf(_ms): a chunk's maps */;
     svfh::PinnedBuf pinned;
 };
 

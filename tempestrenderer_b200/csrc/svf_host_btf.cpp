@@ -97,6 +97,9 @@ svf_status check_btf(svf_ctx* ctx, const svf_btf* btf)
 
 } // namespace
 
+// Decoded samples that svf_error_maps holds at a time (one row at least).
+constexpr size_t kErrorBytes = size_t(512) << 20;
+
 extern "C" {
 
 svf_status svf_btf_probe(const void* file, size_t size, svf_btf_info* info, float* lights_parabolic)
@@ -314,21 +317,27 @@ svf_status svf_error_maps(svf_ctx* ctx, const svf_btf* btf, const svf_svbrdf_map
     SVF_TRY(get_layout(ctx, f.lights_parabolic.data(), f.light_count, &lay));
     const uint64_t N = (uint64_t)f.light_count * f.light_count;
     const size_t row_bytes = sizeof(float) * 3 * N * f.width;
-    size_t free_b = 0, total_b = 0;
-    SVF_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const uint32_t rows = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(h, free_b / 4 / row_bytes));
+    // the decoded rows go by in the context's buffer: a fresh one of 1.3 GB (128 x 128
+    // texels of ring-81) and its release cost 1.9 ms, the whole error 1.5
+    const size_t want = row_bytes * std::max<uint64_t>(1, std::min<uint64_t>(h, kErrorBytes / row_bytes));
+    DevBuf& samples = ctx->btf_decoded;
+    uint32_t rows = (uint32_t)(want / row_bytes);
+    if(samples.n < want)
+    {
+        size_t free_b = 0, total_b = 0;
+        SVF_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        rows = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(rows, (free_b + samples.n) / 4 / row_bytes));
+        SVF_TRY(samples.ensure(row_bytes * rows));
+    }
     const uint32_t nout = color ? 3 : 1;
     const uint32_t sc = maps->sigma_channels;
-    DevBuf samples, md, out;
-    SVF_TRY(samples.ensure(row_bytes * rows));
     const uint64_t rt = (uint64_t)rows * w;
-    SVF_TRY(md.ensure(sizeof(float) * rt * (3 + 3 + sc + 4)));
-    SVF_TRY(out.ensure(sizeof(float) * rt * 2 * nout));
-    float* d_diff = md.as<float>();
+    SVF_TRY(ctx->btf_maps.ensure(sizeof(float) * rt * (3 + 3 + sc + 4 + 2 * nout)));
+    float* d_diff = ctx->btf_maps.as<float>();
     float* d_spec = d_diff + 3 * rt;
     float* d_sig = d_spec + 3 * rt;
     float* d_basis = d_sig + sc * rt;
-    float* d_rmse = out.as<float>();
+    float* d_rmse = d_basis + 4 * rt;
     float* d_psnr = d_rmse + nout * rt;
     for(uint32_t r0 = 0; r0 < h; r0 += rows)
     {
@@ -363,8 +372,8 @@ svf_status svf_error_maps(svf_ctx* ctx, const svf_btf* btf, const svf_svbrdf_map
         SVF_CUDA(svf::launch_error(a, ctx->stream));
         SVF_CUDA(cudaMemcpyAsync(rmse + nout * m0, d_rmse, sizeof(float) * nout * n, cudaMemcpyDefault, ctx->stream));
         SVF_CUDA(cudaMemcpyAsync(psnr + nout * m0, d_psnr, sizeof(float) * nout * n, cudaMemcpyDefault, ctx->stream));
-        SVF_CUDA(cudaStreamSynchronize(ctx->stream));
     }
+    SVF_CUDA(cudaStreamSynchronize(ctx->stream));
     return SVF_OK;
 }
 
@@ -387,8 +396,11 @@ svf_status svf_render_btf(svf_ctx* ctx, const float* lp, uint32_t L, const svf_s
     const size_t texel_bytes = (sample_type == SVF_SAMPLES_F16 ? 2 : 4) * 3 * N;
     bool out_dev = false;
     SVF_TRY(buffer_location(samples, "samples", &out_dev));
-    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(T, (size_t(1) << 30) / texel_bytes));
-    DevBuf md, buf;
+    // device output: as many texels a launch as their maps take 64 MB
+    const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(T, out_dev ? (size_t(64) << 20) / (4 * 13)
+                                                                               : (size_t(1) << 30) / texel_bytes));
+    DevBuf& md = ctx->btf_maps;
+    DevBuf buf;
     SVF_TRY(md.ensure(sizeof(float) * chunk * (3 + 3 + sc + 4)));
     if(!out_dev)
         SVF_TRY(buf.ensure(texel_bytes * chunk));

@@ -114,7 +114,8 @@ svf_status svf_render_btf_ms(svf_ctx* ctx, const float* lp, uint32_t L, const sv
     bool out_dev = false;
     SVF_TRY(buffer_location(samples_out, "samples", &out_dev));
     const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(T, (size_t(1) << 28) / texel_bytes));
-    DevBuf md, buf;
+    DevBuf& md = ctx->btf_maps;
+    DevBuf buf;
     SVF_TRY(md.ensure(sizeof(float) * chunk * (3 + 3 + sc + 4)));
     if(!out_dev)
         SVF_TRY(buf.ensure(texel_bytes * chunk));
