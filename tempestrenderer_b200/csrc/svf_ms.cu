@@ -382,7 +382,11 @@ struct PairEval
         if(depth == 0 || !alive(spec))
             return;
         const M3 cov = covariance(b, mul(sd, sd));
-        const Seen seen0 = seen_from(wo, cov);   // every walk starts along wo
+        // every walk starts along wo; without the table of draws the frame's registers
+        // cost more than it (depth 9: 221 ms a fit against 206)
+        Seen seen0;
+        if constexpr(kTable)
+            seen0 = seen_from(wo, cov);
         float thr[C];
         for(uint32_t s = first; s < samples; ++s)
         {
@@ -391,10 +395,12 @@ struct PairEval
                 thr[c] = spec[c];
             V3 out_l = wo;
             float depth_in = (draws.walk_log() / out_density) * wo.z, dd;
-            scatter(draws, seen0, sd, b, out_l, depth_in, dd);
-            for(uint32_t it = 1;; ++it)
+            if constexpr(kTable)
+                scatter(draws, seen0, sd, b, out_l, depth_in, dd);
+            for(uint32_t it = kTable ? 1 : 0;; ++it)
             {
-                if(depth_in < 0.0f || !event(spec, out_l, depth_in, 4.0f * dd, thr) || it == depth || !alive(thr))
+                if(it > 0 && (depth_in < 0.0f || !event(spec, out_l, depth_in, 4.0f * dd, thr) || it == depth ||
+                              !alive(thr)))
                     break;
                 scatter(draws, seen_from(out_l, cov), sd, b, out_l, depth_in, dd);
             }
@@ -486,6 +492,10 @@ __device__ __forceinline__ V3 direction(const float* geo, uint32_t L, uint32_t d
 }
 
 constexpr int kMsThreads = 256, kWalkThreads = 64;
+// The kernels that walk pair by pair: blocks that share a table of draws are larger.
+// 24 warps an SM either way (80 registers).
+__host__ __device__ constexpr int ms_threads(bool table) { return table ? kMsThreads : 128; }
+__host__ __device__ constexpr int ms_blocks(bool table) { return table ? 3 : 6; }
 constexpr int kRestThreads = 128;
 constexpr uint64_t kRestBlocks = 5 * 148;   // (as many as are resident)
 
@@ -713,7 +723,7 @@ __global__ void __launch_bounds__(kRestThreads) ms_rest_kernel(MsRenderArgs a, M
 // One thread per (texel, view, light), every pair with walks of its own: of few pairs,
 // and where the views' walks have no room.
 template <bool kTable>
-__global__ void __launch_bounds__(kMsThreads) ms_render_kernel(MsRenderArgs a)
+__global__ void __launch_bounds__(ms_threads(kTable), ms_blocks(kTable)) ms_render_kernel(MsRenderArgs a)
 {
     extern __shared__ float4 walk_table[];
     if constexpr(kTable)
@@ -748,11 +758,11 @@ cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk
     auto blocks_of = [](uint64_t n, int threads) { return (n + threads - 1) / threads; };
     if(!walks)
     {
-        const uint64_t blocks = blocks_of(all.count * N, kMsThreads);
+        const uint64_t blocks = blocks_of(all.count * N, ms_threads(smem != 0));
         if(blocks > 0x7fffffffull)
             return cudaErrorInvalidValue;
         if(smem == 0)
-            ms_render_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(all);
+            ms_render_kernel<false><<<(unsigned)blocks, ms_threads(false), 0, stream>>>(all);
         else if((e = allow_smem(ms_render_kernel<true>, smem)) != cudaSuccess)
             return e;
         else
@@ -822,7 +832,7 @@ __device__ __forceinline__ void fd_params(const MsTexel& s, int e, double* p)
 
 // count: the list's length, or (dcount non-null) at most this many, *dcount
 template <bool kTable>
-__global__ void __launch_bounds__(kMsThreads) ms_eval_kernel(MsFitArgs a, uint32_t mode, uint32_t count,
+__global__ void __launch_bounds__(ms_threads(kTable), ms_blocks(kTable)) ms_eval_kernel(MsFitArgs a, uint32_t mode, uint32_t count,
                                                              const uint32_t* dcount)
 {
     extern __shared__ float4 walk_table[];
@@ -1194,19 +1204,20 @@ cudaError_t launch_ms_eval(const MsFitArgs& a, uint32_t mode, uint32_t count, co
         return cudaSuccess;
     const uint64_t N = (uint64_t)a.L * a.L;
     const uint64_t n = (uint64_t)count * N * (mode == kMsEvalJacobian ? kMsEvals : 1);
-    const uint64_t blocks = (n + kMsThreads - 1) / kMsThreads;
+    const size_t smem = walk_table_bytes(kFitWalks, a.bounces);
+    const unsigned threads = ms_threads(smem != 0);
+    const uint64_t blocks = (n + threads - 1) / threads;
     if(blocks > 0x7fffffffull)
         return cudaErrorInvalidValue;
-    const size_t smem = walk_table_bytes(kFitWalks, a.bounces);
     cudaError_t e = cudaSuccess;
     if(smem == 0)
-        ms_eval_kernel<false><<<(unsigned)blocks, kMsThreads, 0, stream>>>(a, mode, count, dcount);
+        ms_eval_kernel<false><<<(unsigned)blocks, threads, 0, stream>>>(a, mode, count, dcount);
     else
     {
         e = allow_smem(ms_eval_kernel<true>, smem);
         if(e != cudaSuccess)
             return e;
-        ms_eval_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(a, mode, count, dcount);
+        ms_eval_kernel<true><<<(unsigned)blocks, threads, smem, stream>>>(a, mode, count, dcount);
     }
     e = cudaGetLastError();
     if(e != cudaSuccess)
