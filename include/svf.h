@@ -320,7 +320,8 @@ typedef struct svf_run_stats
     double   ms_init;           /* default initial guess */
     double   ms_fit;            /* Levenberg-Marquardt */
     double   ms_copy;           /* host<->device staging, when host buffers were given */
-    uint32_t lm_threads;        /* LM kernel configuration the autotuner chose: CTA size */
+    uint32_t lm_threads;        /* LM kernel configuration chosen for the layout: CTA size (the pooled
+                                   kernel's blocks have 256 threads; it sums in this one's order) */
     uint32_t lm_slots;          /* and texels in flight per CTA */
     double   ms_ndf;            /* the NDF GEMM of the default initial guess (part of ms_init) */
     uint32_t graph;             /* svf_fit_texels: 0 launched directly, 1 recorded into a CUDA graph

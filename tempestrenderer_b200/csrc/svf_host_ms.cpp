@@ -120,11 +120,11 @@ svf_status svf_render_btf_ms(svf_ctx* ctx, const float* lp, uint32_t L, const sv
     if(!out_dev)
         SVF_TRY(buf.ensure(texel_bytes * chunk));
     // the views' walks of as many texels as their memory takes; without it (a deep
-    // volume, or no room on the device) every pair walks by itself.  So it does while
-    // all pairs run at once (512 threads an SM): 4 texels of ring-81 take 0.45 ms, 0.91
-    // with the walks shared, whose three kernels each wait for a chain of walks; from
-    // 16 texels on (1.13 against 1.02 ms) sharing is the faster
-    const uint64_t walk_bytes = T * N > (uint64_t)ctx->sms * 512 ? svf::ms_walk_bytes(L, samples, bounces) : 0;
+    // volume, or no room on the device) every pair walks by itself.  So it does for
+    // few pairs, up to 1024 an SM: 4 texels of ring-81 (two events) take 0.47 ms, 0.93
+    // with the walks shared, whose three kernels each wait for a chain of walks; 16
+    // texels 0.82 against 1.03, 25 texels 1.32 against 1.27
+    const uint64_t walk_bytes = T * N > (uint64_t)ctx->sms * 1024 ? svf::ms_walk_bytes(L, samples, bounces) : 0;
     uint64_t walk_texels = walk_bytes ? std::min<uint64_t>(chunk, kMsWalkBytes / walk_bytes) : 0;
     if(walk_texels && ctx->ms_walks.ensure(svf::kMsWalkHeader + walk_bytes * walk_texels) != SVF_OK)
         walk_texels = 0;

@@ -178,13 +178,13 @@ def test_invalid_option_combinations(gpu_ctx, kw):
 
 
 @pytest.mark.parametrize("T,bounces,samples,seed,half", [
-    (90, 1, 256, 0, False), (90, 2, 256, 7, True), (90, 5, 31, 1, False),
+    (160, 1, 256, 0, False), (160, 2, 256, 7, True), (160, 5, 31, 1, False),
     (600, 3, 256, 0, False),    # more texels than the walks' memory holds at a time
-    (80, 8, 256, 0, False),     # too deep for the table of draws
-    (80, 2, 2, 3, False), (80, 0, 16, 0, False)])
+    (160, 8, 256, 0, False),     # too deep for the table of draws
+    (160, 2, 2, 3, False), (160, 0, 16, 0, False)])
 def test_shared_walks_equal_own_walks(gpu_ctx, ms, T, bounces, samples, seed, half):
     """A call of many pairs shares the views' walks, one of few lets every pair walk by
-    itself (at most 512 pairs an SM): bit for bit the same samples."""
+    itself (at most 1024 pairs an SM): bit for bit the same samples."""
     rng = np.random.default_rng(T + bounces)
     q = rng.standard_normal((T, 4)).astype(np.float32)
     q /= np.linalg.norm(q, axis=1, keepdims=True)
