@@ -62,7 +62,7 @@ typedef enum svf_status
 /* per-texel status bits (svf_texel_stats::status) */
 #define SVF_TEXEL_NONFINITE  1u  /* NaN/Inf in the data or the fit; params are the initial guess */
 #define SVF_TEXEL_MAX_ITER   2u  /* stopped at max_iterations */
-#define SVF_TEXEL_TIMEOUT    4u  /* the texel's samples did not arrive (bounded wait expired) */
+#define SVF_TEXEL_TIMEOUT    4u  /* the texel's samples or a pass of its fit did not come (bounded wait expired) */
 
 /* LeastSquaresFitOptions (svbrdf-fitting.hh:100-107) for the supported path */
 #define SVF_LSQ_DIFFUSE      (1u << 1)   /* LSF_OPTON_DIFFUSE: fit the Lambert term (7 parameters);

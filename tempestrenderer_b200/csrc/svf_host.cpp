@@ -238,7 +238,7 @@ svf_status read_error_flag(svf_ctx* ctx, bool with_ndf)
     SVF_CUDA(cudaMemcpyAsync(flag, ctx->error.p, sizeof(flag), cudaMemcpyDeviceToHost, ctx->stream));
     SVF_CUDA(cudaStreamSynchronize(ctx->stream));
     if(flag[0])
-        return fail(SVF_ETIMEOUT, "a bounded device wait expired (a texel slab did not arrive)");
+        return fail(SVF_ETIMEOUT, "a bounded device wait expired (a texel's slab or a pass of its fit did not come)");
     if(with_ndf && flag[2])
         return fail(SVF_ETIMEOUT, "a bounded device wait expired in a tensor-core GEMM");
     return SVF_OK;

@@ -249,17 +249,21 @@ void lm_masks(const svf_lsq_options* o, svf::LmConfig& cfg)
         cfg.fixed_mask |= 0x70u;
 }
 
-// Fault injection for the tests of the bounded slab wait, read from the
+// Fault injection for the tests of the bounded waits, read from the
 // environment at each launch: SVF_FAULT_SKIP_SLAB_COPY=<texel> leaves that
 // texel's slab copy unissued (its wait runs out: SVF_ETIMEOUT, the texel's status
-// SVF_TEXEL_TIMEOUT), SVF_FAULT_WAIT_SPINS=<n> shortens the wait's bound.  No
-// GPU fault is involved: the wait is on a barrier that nothing completes.
+// SVF_TEXEL_TIMEOUT), SVF_FAULT_HOLD_PASS=<texel> leaves that texel's passes in the
+// pooled kernel unopened (the idle warps' wait runs out, with the same status),
+// SVF_FAULT_WAIT_SPINS=<n> shortens the waits' bounds.  No GPU fault is involved:
+// the waits are on a barrier that nothing completes and on a word that nothing sets.
 void lm_fault_injection(svf::LmArgs& a)
 {
-    a.fault_skip_texel = svf::kLmNoFault;
+    a.fault_skip_texel = a.fault_hold_texel = svf::kLmNoFault;
     a.wait_spins = 0;
     if(const char* e = std::getenv("SVF_FAULT_SKIP_SLAB_COPY"))
         a.fault_skip_texel = (uint32_t)std::strtoul(e, nullptr, 10);
+    if(const char* e = std::getenv("SVF_FAULT_HOLD_PASS"))
+        a.fault_hold_texel = (uint32_t)std::strtoul(e, nullptr, 10);
     if(const char* e = std::getenv("SVF_FAULT_WAIT_SPINS"))
         a.wait_spins = (uint32_t)std::strtoul(e, nullptr, 10);
 }
@@ -510,7 +514,7 @@ svf_status svf_lsq_fit_batch_noalloc(const float* lp, uint32_t L, const float* l
     SVF_CUDA(svf::launch_lm_fit_noalloc(lp, L, lum, lum_stride, texels, cfg, init, out, rmse, stats,
                                         static_cast<cudaStream_t>(stream), flags));
     if(flags[0])
-        return fail(SVF_ETIMEOUT, "a bounded device wait expired (a texel slab did not arrive)");
+        return fail(SVF_ETIMEOUT, "a bounded device wait expired (a texel's slab or a pass of its fit did not come)");
     // the status contract of svf_lsq_fit_batch
     if(flags[1])
         return fail(SVF_EPARTIAL, "some texels did not produce a finite fit");

@@ -66,8 +66,10 @@ struct LmArgs
     uint32_t* error_flag;      // set non-zero by a bounded wait that expired
     // Fault injection for tests (the host sets it from the environment): the slab
     // copy of texel fault_skip_texel is not issued, so its wait runs out;
-    // kLmNoFault for none.  wait_spins: the bound of every slab wait (0: default).
-    uint32_t fault_skip_texel;
+    // kLmNoFault for none; the pooled kernel opens no pass of texel fault_hold_texel,
+    // so that its idle warps' waits run out.  wait_spins: the bound of every slab wait
+    // and, but for a floor, of an idle warp's (0: default).
+    uint32_t fault_skip_texel, fault_hold_texel;
     uint32_t wait_spins;
 };
 constexpr uint32_t kLmNoFault = 0xffffffffu;

@@ -688,7 +688,7 @@ cudaError_t launch_lm_fit_noalloc(const float* lights_parabolic, uint32_t L, con
     a.cfg = cfg;
     a.work_counter = flags;
     a.error_flag = flags + 1;
-    a.fault_skip_texel = kLmNoFault;
+    a.fault_skip_texel = a.fault_hold_texel = kLmNoFault;
     a.wait_spins = 0;
     const LmKernelChoice choice = lm_default_choice(L, stride);
     if((e = launch_lm_fit(a, choice, sms, stream)) != cudaSuccess)

@@ -122,13 +122,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
-__device__ __forceinline__ uint64_t global_ns()
-{
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Bounded wait for phase `parity` of `bar` (at most `spins` polls, 0: the
 // default bound); false when the bound expired.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t spins = 0)
@@ -2124,16 +2117,20 @@ struct PoolCtl
 {
     uint32_t sequence;   // passes published
     uint32_t live;       // slots with a texel
-    uint32_t progress;   // shares done (the bound of an idle warp's wait counts waits without progress)
-    uint32_t abort;      // an idle wait ran out: every warp leaves
+    uint32_t progress;   // shares done (the bound of an idle warp's wait counts looks without progress)
+    uint32_t abort;      // an idle wait ran out: every warp that finds nothing to do leaves
     uint32_t epoch;      // phase of `wake`
     uint64_t wake;       // mbarrier, one phase per event an idle warp waits for: shares published, a slot done
     uint32_t open[kPoolMaxSlots];     // a slot's unclaimed shares
     uint32_t number[kPoolMaxSlots];   // and its pass's number among the CTA's passes
 };
 
-constexpr uint64_t kPoolIdleNs = 2000000000ull;   // an idle warp's wait without any progress in the CTA: 2 s
-constexpr uint32_t kPoolNapNs = 500;              // and the time between its looks
+// An idle warp looks every kPoolNapNs at most.  It gives up after as many looks without
+// progress in the CTA as a slab wait has polls, at least kPoolMinLooks (a pass's share or
+// an LM step takes some tens of microseconds; 65536 looks take at least 4 ms).  Looks, not
+// time: a process that is stopped or switched off the GPU makes none.  A slab on its way
+// doesn't count: slot_start bounds that wait.
+constexpr uint32_t kPoolNapNs = 500, kPoolMinLooks = 1u << 16;
 
 template <class M>
 __host__ __device__ constexpr size_t pool_slot_bytes(int nw, uint32_t L, uint64_t stride)
@@ -2175,7 +2172,8 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
             {
                 ctl.number[s] = atomicAdd(&ctl.sequence, 1u);
                 __threadfence_block();
-                atomicExch(&ctl.open[s], (1u << NW) - 1u);
+                if(slot_of(s).texel != args.fault_hold_texel)
+                    atomicExch(&ctl.open[s], (1u << NW) - 1u);
             }
             else
                 atomicSub(&ctl.live, 1u);
@@ -2192,8 +2190,11 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
         ctl.epoch = 0;
         mbar_init(&ctl.wake, 1);
     }
-    if(threadIdx.x < S)
-        ctl.open[threadIdx.x] = 0;   // (every warp looks at every slot from here on)
+    if(threadIdx.x < S)   // (every warp looks at every slot from here on)
+    {
+        ctl.open[threadIdx.x] = 0;
+        slot_of(threadIdx.x).loading = 0;
+    }
     __syncthreads();
     for(uint32_t s = warp; s < S; s += warps)
     {
@@ -2222,7 +2223,7 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
     // lane s watches slot s
     static_assert(kPoolMaxSlots <= 32, "a lane per slot");
     uint32_t seen = 0;
-    uint64_t idle_since = 0;   // 0: not idle
+    uint32_t looks = 0;    // since a share was done; 0: not idle
     bool second = false;   // this is a second look
     for(;;)
     {
@@ -2250,7 +2251,7 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
             second = share == (uint32_t)NW;
             if(second)
                 continue;   // (another scheduler's share, or another warp was faster)
-            idle_since = 0;
+            looks = 0;
             unsigned char* base = smem_raw + s * per_slot;
             float* tab = reinterpret_cast<float*>(base + tab_at);
             double* redd = reinterpret_cast<double*>(base + red_at);
@@ -2289,20 +2290,23 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
         if(__any_sync(0xffffffffu, leave))
             break;
         const uint32_t p = __shfl_sync(0xffffffffu, vctl->progress, 0);
-        const uint64_t now = __shfl_sync(0xffffffffu, global_ns(), 0);
-        if(p != seen || !idle_since)
+        if(p != seen || !looks)
         {
             seen = p;
-            idle_since = now;
+            looks = 1;
         }
-        else if(now - idle_since > kPoolIdleNs)
+        else if(++looks > max(args.wait_spins ? args.wait_spins : kWaitSpins, kPoolMinLooks))
         {
-            if(lane == 0)
+            looks = 0;
+            if(!__any_sync(0xffffffffu, lane < S && *(volatile int*)&slot_of(lane).loading))
             {
-                vctl->abort = 1;
-                atomicOr(args.error_flag, 1u);
+                if(lane == 0)
+                {
+                    vctl->abort = 1;
+                    atomicOr(args.error_flag, 1u);
+                }
+                break;
             }
-            break;
         }
         // suspended until the phase ends, kPoolNapNs at most (a phase of the same
         // parity may have come and gone in between)
@@ -2316,8 +2320,13 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
     __syncthreads();
     if(threadIdx.x == 0)
         for(uint32_t s = 0; s < S; ++s)
-            if(slot_of(s).drain)
-                mbar_wait(&slot_of(s).bar, slot_of(s).parity, args.wait_spins);
+        {
+            Slot<M>& sl = slot_of(s);
+            if(sl.drain)
+                mbar_wait(&sl.bar, sl.parity, args.wait_spins);
+            if(ctl.abort && sl.texel != kNoTexel && args.stats)
+                args.stats[sl.texel].status = SVF_TEXEL_TIMEOUT;   // its pass never came
+        }
 }
 
 using KernelFn = void (*)(LmArgs);
