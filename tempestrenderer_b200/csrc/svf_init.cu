@@ -614,7 +614,7 @@ cudaError_t launch_ndf_operator(const InitLayout& lay, const MeshDevice& mesh, c
     if(e != cudaSuccess)
         return e;
     size_t smem = sizeof(double) * lay.N + ms;
-    e = cudaFuncSetAttribute(ndf_operator_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_all_smem(ndf_operator_kernel);
     if(e != cudaSuccess)
         return e;
     ndf_operator_kernel<<<lay.ndf_rows, 256, smem, stream>>>(mesh, lay.L, lay.N, lay.k_pad, ndf_dirs, row_normals,

@@ -10,6 +10,21 @@
 namespace svf
 {
 
+#ifdef __CUDACC__
+// Lets a launch of k ask for all the shared memory a CTA can have.  The limit is the
+// process's: set to what one launch needs, it may be below what a launch of another
+// thread needs that set its own just before.
+template <typename Kernel>
+cudaError_t allow_all_smem(Kernel* k)
+{
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, k);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   227 * 1024 - (int)at.sharedSizeBytes);
+}
+#endif
+
 // Per-texel LM settings (LevenbergMarquardtCurveFit, include/tempest/math/fitting.hh:457-678).
 struct LmConfig
 {

@@ -750,7 +750,7 @@ cudaError_t launch_luminance(const void* samples, uint32_t sample_type, uint64_t
                                        : LumPass<T, false>::smem(N, lum_stride, hl);
         if(smem > 48 * 1024)
         {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            const cudaError_t e = allow_all_smem(kernel);
             if(e != cudaSuccess)
                 return e;
         }

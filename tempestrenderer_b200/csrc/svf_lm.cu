@@ -2523,7 +2523,7 @@ int lm_max_ctas_per_sm(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool r
     }
     if(!k)
         return 0;
-    if(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if(allow_all_smem(k) != cudaSuccess ||
        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
     {
         cudaGetLastError();
@@ -2559,7 +2559,7 @@ cudaError_t launch_lm_fit(const LmArgs& launch, LmKernelChoice c, int sms, cudaS
         const size_t smem = slots * (rgb ? pool_slot_bytes<RgbModel>(nw, args.L, args.lum_stride)
                                          : pool_slot_bytes<LumModel>(nw, args.L, args.lum_stride));
         args.counter_base = slots * grid;   // the first texels are dealt out
-        if((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        if((e = allow_all_smem(k)) != cudaSuccess)
             return e;
         k<<<grid, 32 * warps, smem, stream>>>(args, slots);
         return cudaGetLastError();
@@ -2569,7 +2569,7 @@ cudaError_t launch_lm_fit(const LmArgs& launch, LmKernelChoice c, int sms, cudaS
     if(!k || per_sm <= 0)
         return cudaErrorInvalidConfiguration;
     const size_t smem = lm_smem_bytes(args.L, args.lum_stride, c, rgb);
-    if((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess ||
+    if((e = allow_all_smem(k)) != cudaSuccess ||
        (e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
         return e;
     args.counter_base = 0;
