@@ -2433,6 +2433,7 @@ uint32_t pool_slots(int nw, uint32_t L, uint64_t stride, bool rgb)
 {
     const size_t per = rgb ? pool_slot_bytes<RgbModel>(nw, L, stride) : pool_slot_bytes<LumModel>(nw, L, stride);
     constexpr size_t kMaxDynamic = 227u * 1024u - 256u;   // (the static part takes PoolCtl)
+    static_assert(sizeof(PoolCtl) <= 256, "PoolCtl in the static part");
     return (uint32_t)std::min<size_t>(kPoolMaxSlots, kMaxDynamic / per);
 }
 
@@ -2499,6 +2500,28 @@ size_t lm_smem_bytes(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool rgb
     return per * (size_t)c.slots;
 }
 
+// The control state a slot counts for in lm_max_ctas_per_sm, luminance and RGB, and a
+// CTA besides.  Constants of the default rule, not sizes to keep up to date: the rule
+// names the number of parts a pass is summed in, so a change moves the bits of fits
+// (tests/test_lm_rule.py has its choices).  They cover the luminance slots of the
+// kernels that the rule can name; the pooled kernel counts its own slots (pool_slots).
+constexpr size_t kRankSlotLum = 1400, kRankSlotRgb = 2168, kRankCta = 16;
+static_assert(sizeof(Slot<LumModel>) <= kRankSlotLum, "a configuration the rule names may not fit on an SM");
+
+// CTAs of a kernel that are resident on an SM; 0: none.
+int resident_ctas(KernelFn k, int threads, size_t smem)
+{
+    int n = 0;
+    if(allow_all_smem(k) != cudaSuccess ||
+       cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
+       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess)
+    {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
 // CTAs of a configuration that fit on an SM; 0: none.  Plain passes: the count the
 // default rule ranks by, CTAs of `threads` threads at 128 registers with `slots`
 // slots of shared memory and control state each (228 KB an SM, 1 KB of it per CTA,
@@ -2515,27 +2538,13 @@ int lm_max_ctas_per_sm(uint32_t L, uint64_t lum_stride, LmKernelChoice c, bool r
     {
         if(!k && (!pool_for(c, false, false, rgb) || pool_slots(c.threads / 32 - 1, L, lum_stride, rgb) == 0))
             return 0;
-        const size_t state = ((rgb ? 2168u : 1400u) * (size_t)c.slots + 16u + 15u) & ~size_t(15);
+        const size_t state = ((rgb ? kRankSlotRgb : kRankSlotLum) * (size_t)c.slots + kRankCta + 15u) & ~size_t(15);
         if(smem + state > 227u * 1024u)
             return 0;
         return (int)std::min<size_t>(65536u / (128u * (size_t)c.threads),
                                      228u * 1024u / (((smem + state + 127) & ~size_t(127)) + 1024u));
     }
-    if(!k)
-        return 0;
-    if(allow_all_smem(k) != cudaSuccess ||
-       cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return 0;
-    }
-    int n = 0;
-    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, c.threads, smem) != cudaSuccess)
-    {
-        cudaGetLastError();
-        return 0;
-    }
-    return n;
+    return k ? resident_ctas(k, c.threads, smem) : 0;
 }
 
 cudaError_t launch_lm_fit(const LmArgs& launch, LmKernelChoice c, int sms, cudaStream_t stream)
@@ -2565,13 +2574,12 @@ cudaError_t launch_lm_fit(const LmArgs& launch, LmKernelChoice c, int sms, cudaS
         return cudaGetLastError();
     }
     KernelFn k = kernel_for(c, fresnel, all_up);
-    const int per_sm = lm_max_ctas_per_sm(args.L, args.lum_stride, c, rgb);
-    if(!k || per_sm <= 0)
+    if(!k)
         return cudaErrorInvalidConfiguration;
     const size_t smem = lm_smem_bytes(args.L, args.lum_stride, c, rgb);
-    if((e = allow_all_smem(k)) != cudaSuccess ||
-       (e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess)
-        return e;
+    const int per_sm = resident_ctas(k, c.threads, smem);   // (sets the kernel's limits too)
+    if(per_sm <= 0)
+        return cudaErrorInvalidConfiguration;
     args.counter_base = 0;
     const uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)per_sm * (uint64_t)sms, args.texels);
     k<<<grid, c.threads, smem, stream>>>(args);
