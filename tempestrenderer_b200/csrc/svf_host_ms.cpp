@@ -142,7 +142,8 @@ svf_status svf_render_btf_ms(svf_ctx* ctx, const float* lp, uint32_t L, const sv
         void* out = out_dev ? static_cast<char*>(samples_out) + c0 * texel_bytes : buf.p;
         svf::MsRenderArgs a{ L, lay->geo.as<float>(), n, d_diff, d_spec, d_sig, d_basis, sc, bounces, samples, seed,
                              sample_type, out };
-        SVF_CUDA(svf::launch_ms_render(a, walk_texels ? ctx->ms_walks.p : nullptr, walk_texels, ctx->stream));
+        SVF_CUDA(svf::launch_ms_render(a, walk_texels ? ctx->ms_walks.p : nullptr, walk_texels, ctx->sms,
+                                       ctx->stream));
         if(!out_dev)
             SVF_CUDA(cudaMemcpyAsync(static_cast<char*>(samples_out) + c0 * texel_bytes, buf.p, texel_bytes * n,
                                      cudaMemcpyDeviceToHost, ctx->stream));

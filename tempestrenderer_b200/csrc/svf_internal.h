@@ -394,7 +394,7 @@ uint64_t ms_walk_bytes(uint32_t L, uint32_t samples, uint32_t bounces);
 constexpr uint64_t kMsWalkHeader = 256;
 // walks: kMsWalkHeader bytes and room for walk_texels texels' walks, or null: every
 // pair walks by itself.
-cudaError_t launch_ms_render(const MsRenderArgs& a, void* walks, uint64_t walk_texels, cudaStream_t stream);
+cudaError_t launch_ms_render(const MsRenderArgs& a, void* walks, uint64_t walk_texels, int sms, cudaStream_t stream);
 
 // The LM state of one texel of the multi-scattering fit (FP64, as the
 // reference's LevenbergMarquardtCurveFit keeps it).

@@ -502,14 +502,14 @@ __device__ __forceinline__ V3 direction(const float* geo, uint32_t L, uint32_t d
 
 constexpr int kMsThreads = 256, kWalkThreads = 64;
 // The kernels that walk pair by pair: blocks that share a table of draws are larger.
-// 24 warps an SM either way (80 registers).
+// 24 warps an SM (80 registers), 16 where the table leaves room for two blocks (6 and 7
+// events: a fit of 24 texels of 40 directions takes 150 and 172 ms with it, 174 and 199
+// without).
 __host__ __device__ constexpr int ms_threads(bool table) { return table ? kMsThreads : 128; }
 __host__ __device__ constexpr int ms_blocks(bool table) { return table ? 3 : 6; }
-constexpr int kRestThreads = 128;
-constexpr uint64_t kRestBlocks = 5 * 148;   // (as many as are resident)
 
-// Shared memory of the walk table; 0 where there is none: past 96 KB two CTAs no longer
-// fit on an SM (256 walks of 7 events take 90 KB).
+// Shared memory of the walk table; 0 where there is none: up to 96 KB (256 walks of 7
+// events take 90 KB), twice of which fits on an SM.
 size_t walk_table_bytes(uint32_t samples, uint32_t depth)
 {
     const uint64_t bytes = sizeof(float4) * walk_draws(samples, depth);
@@ -702,7 +702,14 @@ __global__ void __launch_bounds__(kMsThreads, 4) ms_lookup_kernel(MsRenderArgs a
     store_pair(a, i, f);
 }
 
-__global__ void __launch_bounds__(kRestThreads) ms_rest_kernel(MsRenderArgs a, MsWalks w)
+// Blocks of 128 threads (105 registers) where more than two of them have room for the
+// table; else of 384 at 80 registers, so that two keep the SM busy: 256 texels of ring-81
+// with orientations all over the sphere, 6 and 7 events, take 30.3 and 33.7 ms in all, 39.6
+// and 44.8 in blocks of 128 (32.6 and 34.6 where every pair walks by itself without the
+// table), with orientations near the normal 19.6 and 22.4 (23.0 and 27.4); at 4 events
+// 64 texels take 3.65 ms, 3.94 in blocks of 384.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads > 128 ? 2 : 1) ms_rest_kernel(MsRenderArgs a, MsWalks w)
 {
     extern __shared__ float4 walk_table[];
     const uint32_t lost = *w.lost;
@@ -757,7 +764,7 @@ uint64_t ms_walk_bytes(uint32_t L, uint32_t samples, uint32_t bounces)
     return (uint64_t)L * samples * bounces * (sizeof(float4) + sizeof(float)) + (uint64_t)L * L * sizeof(MsRest);
 }
 
-cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk_texels, cudaStream_t stream)
+cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk_texels, int sms, cudaStream_t stream)
 {
     const uint64_t N = (uint64_t)all.L * all.L;
     if(all.count * N == 0)
@@ -778,8 +785,20 @@ cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk
             ms_render_kernel<true><<<(unsigned)blocks, kMsThreads, smem, stream>>>(all);
         return cudaGetLastError();
     }
-    if((e = allow_smem(ms_walk_kernel, smem)) != cudaSuccess || (e = allow_smem(ms_rest_kernel, smem)) != cudaSuccess)
+    auto rest_kernel = ms_rest_kernel<128>;
+    int rest_threads = 128, resident = 0;
+    if((e = allow_smem(ms_walk_kernel, smem)) != cudaSuccess || (e = allow_smem(rest_kernel, smem)) != cudaSuccess ||
+       (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, rest_kernel, rest_threads, smem)) != cudaSuccess)
         return e;
+    if(resident <= 2)
+    {
+        rest_kernel = ms_rest_kernel<384>;
+        rest_threads = 384;
+        if((e = allow_smem(rest_kernel, smem)) != cudaSuccess ||
+           (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, rest_kernel, rest_threads, smem)) != cudaSuccess)
+            return e;
+    }
+    const uint64_t rest_blocks = (uint64_t)std::max(resident, 1) * sms;   // one wave
     MsWalks w;
     const uint64_t events = walk_texels * all.L * all.samples * all.bounces;
     w.lost = static_cast<uint32_t*>(walks);
@@ -800,8 +819,8 @@ cudaError_t launch_ms_render(const MsRenderArgs& all, void* walks, uint64_t walk
             return cudaErrorInvalidValue;
         ms_walk_kernel<<<(unsigned)views, kWalkThreads, smem, stream>>>(a, w);
         ms_lookup_kernel<<<(unsigned)pairs, kMsThreads, 0, stream>>>(a, w);
-        const uint64_t rest = std::min(blocks_of(a.count * N, kRestThreads), kRestBlocks);
-        ms_rest_kernel<<<(unsigned)rest, kRestThreads, smem, stream>>>(a, w);
+        const uint64_t rest = std::min(blocks_of(a.count * N, rest_threads), rest_blocks);
+        rest_kernel<<<(unsigned)rest, rest_threads, smem, stream>>>(a, w);
         if((e = cudaGetLastError()) != cudaSuccess)
             return e;
     }
