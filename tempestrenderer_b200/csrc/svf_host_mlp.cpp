@@ -149,11 +149,12 @@ svf_status mlp_forward(svf_ctx* ctx, const svf_mlp* mlp, const float* X, int row
         const size_t h = (size_t)r0 * kMlpHidden;
         SVF_CUDA(mlp_gemm(true, r, kMlpHidden, kMlpInputs, X + (size_t)r0 * kMlpInputs, kMlpInputs,
                           w + kMlpW1, kMlpInputs, H1 + h, kMlpHidden, w + kMlpB1, 1, Z1 ? Z1 + h : nullptr, nullptr,
-                          ctx->stream));
+                          ctx->sms, ctx->stream));
         SVF_CUDA(mlp_gemm(true, r, kMlpHidden, kMlpHidden, H1 + h, kMlpHidden, w + kMlpW2, kMlpHidden,
-                          H2 + h, kMlpHidden, w + kMlpB2, 1, Z2 ? Z2 + h : nullptr, nullptr, ctx->stream));
+                          H2 + h, kMlpHidden, w + kMlpB2, 1, Z2 ? Z2 + h : nullptr, nullptr, ctx->sms, ctx->stream));
         SVF_CUDA(mlp_gemm(true, r, kMlpOutputs, kMlpHidden, H2 + h, kMlpHidden, w + kMlpW3, kMlpHidden,
-                          Y + (size_t)r0 * kMlpOutputs, kMlpOutputs, w + kMlpB3, 0, nullptr, nullptr, ctx->stream));
+                          Y + (size_t)r0 * kMlpOutputs, kMlpOutputs, w + kMlpB3, 0, nullptr, nullptr, ctx->sms,
+                          ctx->stream));
     }
     return SVF_OK;
 }
@@ -237,19 +238,19 @@ svf_status mlp_train_step(svf_ctx* ctx, svf_mlp* mlp, MlpScratch& s, const float
     SVF_CUDA(mlp_mse_grad(y, T, rows, kMlpOutputs, dy, s.loss.as<double>(), ctx->stream));
     // layer 3
     SVF_CUDA(mlp_gemm_rows(kMlpOutputs, kMlpHidden, rows, dy, kMlpOutputs, h2, kMlpHidden,
-                      g + kMlpW3, kMlpHidden, ctx->stream));
+                      g + kMlpW3, kMlpHidden, ctx->sms, ctx->stream));
     SVF_CUDA(mlp_colsum(dy, rows, kMlpOutputs, nullptr, nullptr, g + kMlpB3, ctx->stream));
     SVF_CUDA(mlp_gemm(false, rows, kMlpHidden, kMlpOutputs, dy, kMlpOutputs, w + kMlpW3, kMlpHidden,
-                      dh2, kMlpHidden, nullptr, 2, nullptr, z2, ctx->stream));
+                      dh2, kMlpHidden, nullptr, 2, nullptr, z2, ctx->sms, ctx->stream));
     // layer 2
     SVF_CUDA(mlp_gemm_rows(kMlpHidden, kMlpHidden, rows, dh2, kMlpHidden, h1, kMlpHidden,
-                      g + kMlpW2, kMlpHidden, ctx->stream));
+                      g + kMlpW2, kMlpHidden, ctx->sms, ctx->stream));
     SVF_CUDA(mlp_colsum(dh2, rows, kMlpHidden, nullptr, nullptr, g + kMlpB2, ctx->stream));
     SVF_CUDA(mlp_gemm(false, rows, kMlpHidden, kMlpHidden, dh2, kMlpHidden, w + kMlpW2, kMlpHidden,
-                      dh1, kMlpHidden, nullptr, 2, nullptr, z1, ctx->stream));
+                      dh1, kMlpHidden, nullptr, 2, nullptr, z1, ctx->sms, ctx->stream));
     // layer 1
     SVF_CUDA(mlp_gemm_rows(kMlpHidden, kMlpInputs, rows, dh1, kMlpHidden, X, kMlpInputs, g + kMlpW1,
-                      kMlpInputs, ctx->stream));
+                      kMlpInputs, ctx->sms, ctx->stream));
     SVF_CUDA(mlp_colsum(dh1, rows, kMlpHidden, nullptr, nullptr, g + kMlpB1, ctx->stream));
     ++mlp->step;
     SVF_CUDA(mlp_adam(w, g, mlp->m.as<float>(), mlp->v.as<float>(), kMlpParams, lr, mlp->step, sgd, ctx->stream));

@@ -274,12 +274,12 @@ constexpr size_t kMlpW3 = kMlpB2 + kMlpHidden, kMlpB3 = kMlpW3 + (size_t)kMlpOut
 constexpr size_t kMlpParams = kMlpB3 + kMlpOutputs;
 
 // C[M][N] = op(A) op(B) (+ bias[n]); mode 1: Z = C (if Z), C = gelu(C); mode 2:
-// C *= gelu'(Zin).  FP32 (training).
+// C *= gelu'(Zin).  FP32 (training).  sms: of the device (the tiles' sizes follow it, the sums don't)
 cudaError_t mlp_gemm(bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                     const float* bias, int mode, float* Z, const float* Zin, cudaStream_t stream);
+                     const float* bias, int mode, float* Z, const float* Zin, int sms, cudaStream_t stream);
 // C [M][N] = A^T B over K rows (the weight gradients); widths multiples of 4, 16-byte aligned operands
 cudaError_t mlp_gemm_rows(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                          cudaStream_t stream);
+                          int sms, cudaStream_t stream);
 cudaError_t mlp_colsum(const float* X, int M, int N, double* sum, double* sumsq, float* sum_f, cudaStream_t stream);
 cudaError_t mlp_normalize(float* X, int M, int N, const float* mean, const float* rstd, cudaStream_t stream);
 cudaError_t mlp_mse_grad(const float* Y, const float* T, int M, int N, float* dY, double* loss, cudaStream_t stream);

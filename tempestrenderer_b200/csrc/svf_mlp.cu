@@ -660,11 +660,11 @@ cudaError_t launch_gemm(int M, int N, int K, const float* A, int lda, const floa
 // Tiles: a column of 8 outputs (the network's last layer) takes 8-wide tiles; else
 // 64 x 64 while they make a CTA for every SM, 32 x 32 below.
 template <bool kTB, class... Args>
-cudaError_t pick_gemm(int M, int N, Args... args)
+cudaError_t pick_gemm(int sms, int M, int N, Args... args)
 {
     if(N <= 8)
         return launch_gemm<kTB, 32, 8, 1, 1>(M, N, args...);
-    if((int64_t)((M + 63) / 64) * ((N + 63) / 64) >= 148)
+    if((int64_t)((M + 63) / 64) * ((N + 63) / 64) >= sms)
         return launch_gemm<kTB, 64, 64, 4, 4>(M, N, args...);
     return launch_gemm<kTB, 32, 32, 2, 4>(M, N, args...);
 }
@@ -686,22 +686,22 @@ cudaError_t launch_rows(int M, int N, int K, const float* A, int lda, const floa
 } // namespace
 
 cudaError_t mlp_gemm(bool tb, int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                     const float* bias, int mode, float* Z, const float* Zin, cudaStream_t stream)
+                     const float* bias, int mode, float* Z, const float* Zin, int sms, cudaStream_t stream)
 {
-    return tb ? pick_gemm<true>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream)
-              : pick_gemm<false>(M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream);
+    return tb ? pick_gemm<true>(sms, M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream)
+              : pick_gemm<false>(sms, M, N, K, A, lda, B, ldb, C, ldc, bias, mode, Z, Zin, stream);
 }
 
 cudaError_t mlp_gemm_rows(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc,
-                          cudaStream_t stream)
+                          int sms, cudaStream_t stream)
 {
     if(M % 4 || N % 4 || lda % 4 || ldb % 4 || (reinterpret_cast<uintptr_t>(A) & 15u) ||
        (reinterpret_cast<uintptr_t>(B) & 15u))
         return cudaErrorInvalidValue;   // (the 16-byte copies; every layer's widths are multiples of 8)
     // the largest tile that makes a CTA for at least half the SMs
-    if((int64_t)M * N >= 148 * 16 * 32 / 2)
+    if((int64_t)M * N >= (int64_t)sms * 16 * 32 / 2)
         return launch_rows<16, 32, 2, 2>(M, N, K, A, lda, B, ldb, C, ldc, stream);
-    if((int64_t)M * N >= 148 * 16 * 16 / 2)
+    if((int64_t)M * N >= (int64_t)sms * 16 * 16 / 2)
         return launch_rows<16, 16, 2, 2>(M, N, K, A, lda, B, ldb, C, ldc, stream);
     return launch_rows<8, 8, 1, 1>(M, N, K, A, lda, B, ldb, C, ldc, stream);
 }
