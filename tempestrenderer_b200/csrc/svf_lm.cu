@@ -2170,10 +2170,11 @@ __global__ void __launch_bounds__(32 * kPoolWarps, 1) lm_pool_kernel(LmArgs args
         {
             if(build)
             {
+                // (ahead of the atomics: between them the read took 0.6 % of an RGB fit)
+                const uint32_t shares = slot_of(s).texel != args.fault_hold_texel ? (1u << NW) - 1u : 0u;
                 ctl.number[s] = atomicAdd(&ctl.sequence, 1u);
                 __threadfence_block();
-                if(slot_of(s).texel != args.fault_hold_texel)
-                    atomicExch(&ctl.open[s], (1u << NW) - 1u);
+                atomicExch(&ctl.open[s], shares);
             }
             else
                 atomicSub(&ctl.live, 1u);
