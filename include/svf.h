@@ -31,6 +31,12 @@
  *     which.  Host buffers are staged through pinned memory in chunks.  A
  *     sample or output buffer in device memory of another GPU is rejected with
  *     SVF_EINVAL before anything is launched.
+ *   - A context keeps the device memory its calls worked in, for the next call,
+ *     until svf_destroy.  Besides the fits' chunks: svf_error_maps the samples it
+ *     decodes, at most 512 MB or one row of texels, if that is larger (shared with
+ *     svf_fit_btf's chunk); svf_render_btf_ms the views' walks, at most 256 MB; both
+ *     and svf_render_btf the maps of a chunk's texels, at most 64 MB at 16 or more
+ *     directions.
  *
  * Errors are returned as svf_status codes; no exception crosses the ABI.
  * svf_last_error() gives a message for the calling thread's last failure.
@@ -320,9 +326,12 @@ typedef struct svf_run_stats
     double   ms_init;           /* default initial guess */
     double   ms_fit;            /* Levenberg-Marquardt */
     double   ms_copy;           /* host<->device staging, when host buffers were given */
-    uint32_t lm_threads;        /* LM kernel configuration chosen for the layout: CTA size (the pooled
-                                   kernel's blocks have 256 threads; it sums in this one's order) */
-    uint32_t lm_slots;          /* and texels in flight per CTA */
+    uint32_t lm_threads;        /* LM configuration the layout's rule names: a pass is summed in
+                                   lm_threads / 32 - 1 parts.  The CTA size of luminance fits of 2 to 4
+                                   parts; RGB fits and luminance fits of 7 parts run in the pooled
+                                   kernel, one CTA an SM of up to 256 threads */
+    uint32_t lm_slots;          /* and texels in flight per CTA (pooled: as many as its shared memory
+                                   holds, at most 16) */
     double   ms_ndf;            /* the NDF GEMM of the default initial guess (part of ms_init) */
     uint32_t graph;             /* svf_fit_texels: 0 launched directly, 1 recorded into a CUDA graph
                                    and launched, 2 replayed (a repeat of the previous call) */
