@@ -20,7 +20,7 @@
 // its samples leave with their channels together and two CTAs share an SM (one
 // stores while the other multiplies).  What bounds it is the 32 words a clock that
 // shared memory returns to registers, whether or not lanes ask for the same word: 12
-// words for 32 products, 82 % of that rate against 55 % of the FP32 pipe's.  8 x 8 a
+// words for 32 products, 82 % of that rate against 51 % of the FP32 pipe's.  8 x 8 a
 // thread (16 words for 64 products) needs 192 sums and leaves one CTA: 9.25 ms where
 // this takes 8.45.  Half planes accumulate with FMAs (a product of two halves is exact
 // in float, so the FMA rounds as the reference's separate multiply and add do), two

@@ -2092,9 +2092,9 @@ __global__ void __launch_bounds__(32 * (NW + 1), kPass == kPassPacked ? 1 : min_
 // workers to a scheduler and one beside the control warp.  Measured against it:
 // RGB LM of 173 x 173 ring-81 texels 25.4 -> 18.9 ms, 97 x 97 Fibonacci-151 texels
 // 8.88 -> 8.17 ms.  On ring-81 luminance slabs, 7 slots of 4 shares here and three
-// CTAs of 4 workers there, both keep the SM's FP32 pipe at what its operand reads
-// allow (400 x 400: 46.3 and 46.8 ms), and the shorter launches end later here
-// (150 x 150: 7.6 and 7.4 ms), so those stay where they were.
+// CTAs of 4 workers there take the same time (400 x 400: 46.3 and 46.8 ms), and the
+// shorter launches end later here (150 x 150: 7.6 and 7.4 ms), so those stay where
+// they were.
 //
 // Slot hand-over (all in shared memory): the table, constants and slab of a slot
 // are complete, then its sequence number, then a fence, then its shares' bits in
@@ -2106,11 +2106,12 @@ __global__ void __launch_bounds__(32 * (NW + 1), kPass == kPassPacked ? 1 : min_
 // share of its scheduler, u = (warp - s) mod 4 (the SM deals a CTA's warps to its
 // four schedulers in turn), and another one only on a second look, so that the
 // shares of the few texels a launch ends with spread over the schedulers.
-// Two warps a scheduler, with all the registers they ask for (luminance 180, RGB
-// 255): a pass's steps are bound by the FP32 pipe's operand reads (luminance: 225
-// cycles a step and scheduler with two warps on it, 200 with four), so that more
-// warps at 128 registers gain little and lose by what they spill (RGB, 173 x 173:
-// 23.0 ms with 16 warps, 18.9 with 8; Fibonacci-151, 97 x 97: 10.4 and 8.2 ms).
+// Two warps a scheduler, with all the registers they ask for (luminance 186, RGB
+// 255).  They keep the FMA pipe 62 % busy and 61 % of the issue slots used (97 x 97
+// Fibonacci-151 texels; RGB, 97 x 97 ring-81: 39 and 56 %, with waits for
+// instructions), bound by the latency of results that two warps don't cover; more
+// warps at 128 registers lose more by what they spill (RGB, 173 x 173: 23.0 ms with 16
+// warps, 18.9 with 8; Fibonacci-151, 97 x 97: 10.4 and 8.2 ms).
 constexpr int kPoolWarps = 8, kPoolMaxSlots = 16;
 
 struct PoolCtl

@@ -586,8 +586,8 @@ __device__ __forceinline__ void store_pair(const MsRenderArgs& a, uint64_t i, co
 // (ms_lookup_kernel); a pair that loses sight of an event that its view's walk goes on
 // from leaves its sums in a list, and the rest of its walks are its own
 // (ms_rest_kernel).  16 x 16 texels of ring-81, 256 walks of two events: 0.31 + 4.0 +
-// 1.1 ms, where every pair walking by itself (ms_render_kernel) takes 10.3, and 16.1
-// without the table of draws.  Finishing the lost pairs in the lookup takes 9.9: a few
+// 1.1 to 1.4 ms (by the maps), where every pair walking by itself (ms_render_kernel)
+// takes 10.0, and 16.0 without the table of draws.  Finishing the lost pairs in the lookup takes 9.9: a few
 // lanes of a warp then walk for all, on half as many warps.
 struct MsRest
 {
